@@ -244,6 +244,28 @@ SHIP_SHAPES = [
 SHIP_GROUPED = [(512, 0, ("ffma", "bf16x6", "bf16x3"))]
 
 
+def prefer_library(entry: dict, m: int, n: int, k: int, variant: str, steps: int = 5) -> dict:
+    """`entry` with the library's own choice in place of a tuned schedule that
+    beats it by less than 2 % on the tuned shape: a shape class spans a factor
+    of two in every dimension, and the library's choice follows the shape
+    inside it (its time is kept in "library_ms")."""
+    import torch
+
+    from .sgemm import gemm, gemm_workspace_size
+    library = {"tile": 0, "split_k": 0, "chunk_k": 0, "raster_group": 0}
+    g = torch.Generator(device="cuda").manual_seed(1)
+    A = torch.rand((m, k), device="cuda", generator=g) * 2 - 1
+    B = torch.rand((k, n), device="cuda", generator=g) * 2 - 1
+    C = torch.empty((m, n), device="cuda")
+    ws = torch.empty(max(gemm_workspace_size(m, n, k, variant, library), 256), dtype=torch.uint8,
+                     device="cuda")
+    ms = _time(lambda: gemm(A, B, C, variant=variant, config=library, workspace=ws), steps)
+    out = dict(entry, library_ms=ms)
+    if ms <= 1.02 * entry["ms"]:
+        out["config"] = library
+    return out
+
+
 def ship(path: str = SHIPPED_PATH, steps: int = 3) -> dict:
     """Tune every shipped shape class on the current GPU and write the table
     (with each candidate's measured time as evidence) to `path`."""
@@ -253,10 +275,11 @@ def ship(path: str = SHIPPED_PATH, steps: int = 3) -> dict:
     out = {}
     for (m, n, k), variants in SHIP_SHAPES:
         for v in variants:
-            cfg = tune(m, n, k, v, steps=steps, max_candidates=64, store=False)
-            out[shape_key(m, n, k, v)] = _last_entry
-            print(json.dumps({"shape": [m, n, k], "variant": v, "config": cfg,
-                              "ms": _last_entry["ms"]}), flush=True)
+            tune(m, n, k, v, steps=steps, max_candidates=64, store=False)
+            e = prefer_library(_last_entry, m, n, k, v, steps)
+            out[shape_key(m, n, k, v)] = e
+            print(json.dumps({"shape": [m, n, k], "variant": v, "config": e["config"],
+                              "ms": e["ms"], "library_ms": e["library_ms"]}), flush=True)
             torch.cuda.empty_cache()
     for count, seed, variants in SHIP_GROUPED:
         dims = sweep.grouped_dims(count, seed)

@@ -260,7 +260,7 @@ static int gemm_dispatch(int trans_a, int trans_b, int M, int N, int K, const fl
 
   if (variant == HBSG_FFMA) {
     if (tile >= ffma_num_tiles()) return HBSG_ERR_UNSUPPORTED;
-    if (tile < 0) tile = ffma_pick_tile(M, N, K, batch, sms);
+    if (tile < 0) tile = ffma_pick_tile(M, N, K, batch, sms, trans_a || trans_b);
     int splits = cfg && cfg->split_k > 1 ? cfg->split_k : 1;
     if (splits > 1 && K == 0) splits = 1;
     const size_t need = ffma_workspace_bytes(M, N, batch, splits);

@@ -5,22 +5,28 @@
 // round-robin (kernel.cpp:300-302), streams 16x16 blocks of A and B from DRAM
 // into scratchpad (load_block, kernel.cpp:36-109) and runs a 4x4
 // register-blocked fmaf chain over k (compute_block, kernel.cpp:186-275).
-// Here one CTA owns a BM x BN output tile; A and B tiles stream from HBM into
-// a STAGES-deep shared-memory ring with 16-byte cp.async (zero-filled at the
-// matrix edges), and each thread owns a TM x TN register block that it
-// updates with one fused multiply-add per k in ascending k. The arithmetic
-// per output element is therefore exactly the reference device kernel's:
+// Here one CTA owns a BM x BN output tile: a producer warpgroup streams A and
+// B tiles from HBM into a STAGES-deep shared-memory ring with cp.async
+// (zero-filled past K), and each thread of the compute warps owns a TM x TN
+// register block that it updates with one fused multiply-add per k in
+// ascending k. The arithmetic per output element is therefore exactly the
+// reference device kernel's:
 // acc = 0.0f; for k = 0..K-1: acc = fmaf(a[m][k], b[k][n], acc).
 //
-// Layout in shared memory (per stage):
-//   A: BM rows x (BK + 4) floats, k contiguous. The +4 pad makes 8
-//      consecutive rows fall in 8 distinct 16-byte bank groups, so the
-//      8 distinct rows read by a quarter-warp with LDS.128 are conflict-free.
-//   B: BK rows x BN floats, n contiguous.
-// Thread layout inside a warp: lane = tn*8 + tm (tm < 8, tn < 4). Thread
-// (tm, tn) owns rows {tm + 8i} and columns {16j + 4tn + c} of its warp tile:
-// a quarter-warp reads 8 distinct A rows (no conflict) and one B float4
-// (broadcast); the whole warp reads 64 contiguous bytes of B.
+// Layout in shared memory (per stage): BK rows of BM floats of A and BK rows
+// of BN floats of B, m and n contiguous (an operand that is k-contiguous in
+// memory is transposed on the way in, ffma_kernel.cuh).
+// Thread layout inside a compute warp: lane = tn*8 + tm (tm < 8, tn < 4).
+// Thread (tm, tn) owns rows {32i + 4tm + c} and columns {16j + 4tn + c}: the
+// warp's fragment of one k is 128 contiguous bytes of A per i and 64 of B per
+// j, read as 16-byte vectors without bank conflicts.
+//
+// What bounds it: the FMA pipe (a packed FMA holds it two cycles), once the
+// loads are out of the FMA stream. 4096^3: 2.66 -> 2.23 ms (51.7 -> 61.5
+// TFLOP/s, 0.87 of the measured packed-FMA roof) against the form whose
+// compute warps issued the loads between two barriers per k-tile; two
+// 512^3 products 24.6 -> 18.4 us; 1531 x 1009 x 2047 with A transposed and
+// unaligned 239 -> 152 us.
 #include "ffma_kernel.cuh"
 
 namespace hbsg {
@@ -57,9 +63,17 @@ __global__ void __launch_bounds__(FfmaShape<BM, BN, BK, WM, WN, STAGES>::kThread
     ldc = p.ldc;
     vec_store = p.vec_store;
   }
-  ffma_tile<BM, BN, BK, WM, WN, STAGES, VEC, PAIR, TA, TB>(p.A + batch * p.strideA, p.lda,
-                                                   p.B + batch * p.strideB, p.ldb, p.M, p.N,
-                                                   k_begin, k_end, m0, n0, C, ldc, vec_store, smem);
+  using S = FfmaShape<BM, BN, BK, WM, WN, STAGES>;
+  if (threadIdx.x >= S::kCompute) {
+    ffma_regs_dec<S::kProducerRegs>();
+    ffma_produce<S, BM, BN, BK, STAGES, VEC, TA, TB>(p.A + batch * p.strideA, p.lda,
+                                                     p.B + batch * p.strideB, p.ldb, p.M, p.N,
+                                                     k_begin, k_end, m0, n0, smem);
+  } else {
+    ffma_regs_inc<S::kComputeRegs>();
+    ffma_compute<S, BM, BN, BK, WM, WN, STAGES, PAIR, TA, TB>(p.M, p.N, k_begin, k_end, m0, n0, C,
+                                                              ldc, vec_store, smem);
+  }
 }
 
 // Fixed-order reduction of split-K partial slices: C = ((p0 + p1) + p2) + ...
@@ -92,37 +106,45 @@ struct FfmaEntry {
 template <int BM, int BN, int BK, int WM, int WN, int STAGES, bool PAIR>
 static cudaError_t launch_ffma(const FfmaParams& p, dim3 grid, cudaStream_t st, bool vec) {
   using S = FfmaShape<BM, BN, BK, WM, WN, STAGES>;
+  constexpr int smem = S::smem_bytes(false, false);
   auto kv = ffma_sgemm_kernel<BM, BN, BK, WM, WN, STAGES, true, PAIR>;
   auto ks = ffma_sgemm_kernel<BM, BN, BK, WM, WN, STAGES, false, PAIR>;
   auto k = vec ? kv : ks;
   static uint64_t mask_v = 0, mask_s = 0;
-  if (!set_smem_once(reinterpret_cast<const void*>(k), S::kSmemBytes, vec ? &mask_v : &mask_s))
+  static int regs_v = 0, regs_s = 0;
+  if (!set_smem_once(reinterpret_cast<const void*>(k), smem, vec ? &mask_v : &mask_s))
     return cudaErrorInvalidValue;
-  k<<<grid, S::kThreads, S::kSmemBytes, st>>>(p);
+  if (!ffma_regs_ok<S>(reinterpret_cast<const void*>(k), vec ? &regs_v : &regs_s))
+    return cudaErrorInvalidConfiguration;
+  k<<<grid, S::kThreads, smem, st>>>(p);
   return cudaGetLastError();
 }
 
-// Transposed-operand kernels (4-byte copy path) for a tile shape.
-template <int BM, int BN, int BK, int WM, int WN, int STAGES>
+// Transposed-operand kernels for a tile shape.
+template <int BM, int BN, int BK, int WM, int WN, int STAGES, bool VEC>
 static cudaError_t launch_ffma_trans(const FfmaParams& p, dim3 grid, cudaStream_t st, int ta,
                                      int tb) {
   using S = FfmaShape<BM, BN, BK, WM, WN, STAGES>;
-  auto k10 = ffma_sgemm_kernel<BM, BN, BK, WM, WN, STAGES, false, true, true, false>;
-  auto k01 = ffma_sgemm_kernel<BM, BN, BK, WM, WN, STAGES, false, true, false, true>;
-  auto k11 = ffma_sgemm_kernel<BM, BN, BK, WM, WN, STAGES, false, true, true, true>;
+  auto k10 = ffma_sgemm_kernel<BM, BN, BK, WM, WN, STAGES, VEC, true, true, false>;
+  auto k01 = ffma_sgemm_kernel<BM, BN, BK, WM, WN, STAGES, VEC, true, false, true>;
+  auto k11 = ffma_sgemm_kernel<BM, BN, BK, WM, WN, STAGES, VEC, true, true, true>;
   auto k = ta && tb ? k11 : ta ? k10 : k01;
   static uint64_t masks[3] = {0, 0, 0};
+  static int regs[3] = {0, 0, 0};
   const int slot = ta && tb ? 2 : ta ? 0 : 1;
-  if (!set_smem_once(reinterpret_cast<const void*>(k), S::kSmemBytes, &masks[slot]))
+  const int smem = S::smem_bytes(ta != 0, tb != 0);
+  if (!set_smem_once(reinterpret_cast<const void*>(k), smem, &masks[slot]))
     return cudaErrorInvalidValue;
-  k<<<grid, S::kThreads, S::kSmemBytes, st>>>(p);
+  if (!ffma_regs_ok<S>(reinterpret_cast<const void*>(k), &regs[slot]))
+    return cudaErrorInvalidConfiguration;
+  k<<<grid, S::kThreads, smem, st>>>(p);
   return cudaGetLastError();
 }
 
 #define HBSG_FFMA_ENTRY(BM, BN, BK, WM, WN, ST, PAIR)                                   \
   FfmaEntry {                                                                           \
     BM, BN, BK, WM, WN, ST, FfmaShape<BM, BN, BK, WM, WN, ST>::kThreads,                \
-        FfmaShape<BM, BN, BK, WM, WN, ST>::kSmemBytes,                                  \
+        FfmaShape<BM, BN, BK, WM, WN, ST>::smem_bytes(false, false),                    \
         FfmaShape<BM, BN, BK, WM, WN, ST>::kMinBlocks,                                  \
         &launch_ffma<BM, BN, BK, WM, WN, ST, PAIR>                                      \
   }
@@ -130,11 +152,11 @@ static cudaError_t launch_ffma_trans(const FfmaParams& p, dim3 grid, cudaStream_
 static const FfmaEntry kFfmaTiles[] = {
     HBSG_FFMA_ENTRY(128, 128, 16, 64, 64, 4, true),   // 1: 4 warps, 2 CTAs/SM, packed FMA
     HBSG_FFMA_ENTRY(128, 256, 16, 64, 64, 4, true),   // 2: 8 warps, packed FMA
-    HBSG_FFMA_ENTRY(64, 64, 16, 32, 32, 4, true),     // 3: 4 warps, small problems
+    HBSG_FFMA_ENTRY(64, 64, 16, 32, 32, 6, true),     // 3: 4 warps, small problems
     HBSG_FFMA_ENTRY(128, 64, 16, 64, 32, 4, true),    // 4: 4 warps, narrow N
     HBSG_FFMA_ENTRY(128, 256, 32, 64, 64, 3, true),   // 5: 8 warps, deeper K tile
     HBSG_FFMA_ENTRY(256, 128, 16, 64, 64, 4, true),   // 6: 8 warps, tall
-    HBSG_FFMA_ENTRY(128, 128, 32, 64, 64, 3, true),   // 7: 4 warps, deeper K tile
+    HBSG_FFMA_ENTRY(128, 128, 32, 64, 64, 2, true),   // 7: 4 warps, deeper K tile
     HBSG_FFMA_ENTRY(128, 128, 16, 64, 64, 4, false),  // 8: as 1 with scalar FMA
     HBSG_FFMA_ENTRY(128, 128, 16, 64, 32, 4, true),   // 9: 8 warps, 8x8 per thread
 };
@@ -155,32 +177,42 @@ bool ffma_tile_info(int idx, hbsg_tile_info* out) {
   return true;
 }
 
-// Pick the tile with the best estimated SM utilisation, preferring the large
-// tile when the wave count is high (fewer bytes per flop).
-int ffma_pick_tile(int M, int N, int K, int batch, int num_sms) {
-  (void)K;
-  double best = -1.0;
-  int best_idx = 0;
-  const int cand[] = {0, 1, 3, 2};  // 128x128, 128x256, 128x64, 64x64
-  for (int idx : cand) {
-    const FfmaEntry& e = kFfmaTiles[idx];
+// Tile for an M x N x K product (or a batch of them): the least estimated
+// time of the SM that gets the most tiles. An SM's tiles run `res` at a time;
+// the rates are those measured with 1 and with `res` tiles of a shape on every
+// SM (TFLOP/s over 148 SMs, K = 4096, packed FMA), so a grid that leaves each
+// SM one small tile, a ragged last round and the padding of edge tiles are
+// all charged. 1536 x 1024 x 2048 takes 64 x 64 tiles (three per SM at most,
+// 150 us) rather than 128 x 128 (one on 96 of the SMs, 177 us); 4096^3 takes
+// 128 x 128 (2.24 ms). Transposed operands have kernels for two of the shapes.
+int ffma_pick_tile(int M, int N, int K, int batch, int num_sms, bool trans) {
+  struct Rate {
+    int idx, res;
+    double one, full;
+  };
+  static const Rate kRates[] = {
+      {0, 2, 57.0, 62.1},  // 128 x 128
+      {1, 1, 62.4, 62.4},  // 128 x 256
+      {3, 2, 51.0, 54.8},  // 128 x 64
+      {2, 3, 41.8, 50.7},  // 64 x 64
+  };
+  constexpr double kTileUs = 1.5;  // first loads and the stores of a tile
+  double best = 0.0;
+  int best_idx = -1;
+  for (const Rate& r : kRates) {
+    if (trans && r.idx != 0 && r.idx != 2) continue;
+    const FfmaEntry& e = kFfmaTiles[r.idx];
     const long tiles = (long)((M + e.bm - 1) / e.bm) * ((N + e.bn - 1) / e.bn) * batch;
-    const int per_sm = e.per_sm;
-    const double slots = (double)num_sms * per_sm;
-    const double waves = tiles / slots;
-    const double eff = waves / ceil(waves);  // tail efficiency
-    // work per tile relative to the biggest tile: bigger tiles amortise loads
-    // measured at 8192^3: 128x128 (2 CTAs/SM) is the fastest shape
-    const double tile_eff = (e.bm * e.bn == 128 * 128) ? 1.0 : (e.bm * e.bn >= 128 * 256 ? 0.96 : 0.85);
-    const double fill = fmin(1.0, tiles / slots);
-    // share of the tile's rows and columns inside the matrix (a 128-wide tile
-    // on N = 64 computes twice the columns it stores)
-    const double inside = (double)M / (((M + e.bm - 1) / e.bm) * e.bm) *
-                          ((double)N / (((N + e.bn - 1) / e.bn) * e.bn));
-    const double score = eff * tile_eff * (fill < 1.0 ? fill : 1.0) * inside;
-    if (score > best + 1e-9) {
-      best = score;
-      best_idx = idx;
+    const long per_sm = (tiles + num_sms - 1) / num_sms;
+    const long rounds = per_sm / r.res, rest = per_sm % r.res;
+    const double us = 2.0 * e.bm * e.bn * (K > 0 ? K : 1) * 148.0 * 1e-6;  // x 1 / TFLOP/s
+    const double rest_rate =
+        r.res > 1 ? r.one + (r.full - r.one) * (rest - 1) / (r.res - 1) : r.full;
+    double t = rounds * (r.res * us / r.full + kTileUs);
+    if (rest > 0) t += rest * us / rest_rate + kTileUs;
+    if (best_idx < 0 || t < best) {
+      best = t;
+      best_idx = r.idx;
     }
   }
   return best_idx;
@@ -212,7 +244,7 @@ cudaError_t ffma_launch(int tile_idx, FfmaParams p, int batch, int sms, cudaStre
   } else {
     p.k_per_split = p.K;
   }
-  const bool vec = !ta && !tb && ((p.lda & 3) == 0) && ((p.ldb & 3) == 0) &&
+  const bool vec = ((p.lda & 3) == 0) && ((p.ldb & 3) == 0) &&
                    ((reinterpret_cast<uintptr_t>(p.A) & 15) == 0) &&
                    ((reinterpret_cast<uintptr_t>(p.B) & 15) == 0) && ((p.strideA & 3) == 0) &&
                    ((p.strideB & 3) == 0);
@@ -221,8 +253,12 @@ cudaError_t ffma_launch(int tile_idx, FfmaParams p, int batch, int sms, cudaStre
   dim3 grid((unsigned)(p.tiles_m * p.tiles_n), (unsigned)p.splits, (unsigned)batch);
   cudaError_t err;
   if (ta || tb) {
-    err = tile_idx == 0 ? launch_ffma_trans<128, 128, 16, 64, 64, 4>(p, grid, st, ta, tb)
-                        : launch_ffma_trans<64, 64, 16, 32, 32, 4>(p, grid, st, ta, tb);
+    if (tile_idx == 0)
+      err = vec ? launch_ffma_trans<128, 128, 16, 64, 64, 4, true>(p, grid, st, ta, tb)
+                : launch_ffma_trans<128, 128, 16, 64, 64, 4, false>(p, grid, st, ta, tb);
+    else
+      err = vec ? launch_ffma_trans<64, 64, 16, 32, 32, 6, true>(p, grid, st, ta, tb)
+                : launch_ffma_trans<64, 64, 16, 32, 32, 6, false>(p, grid, st, ta, tb);
   } else {
     err = e.launch(p, grid, st, vec);
   }

@@ -367,23 +367,41 @@ __global__ void __launch_bounds__(FfmaShape<BM, BN, BK, WM, WN, STAGES>::kThread
                         int* __restrict__ queue) {
   // Tiles are claimed from `queue` (zeroed before the launch): thread 0 claims
   // the next tile when a tile starts, so the atomic's latency overlaps it.
+  // Producers and compute warps (ffma_kernel.cuh) walk the same sequence of
+  // tiles; both meet at barrier 0 twice between tiles (the tile's last reads
+  // of the ring and of s_next are done; s_next is written).
+  using S = FfmaShape<BM, BN, BK, WM, WN, STAGES>;
   extern __shared__ __align__(16) float smem[];
-  __shared__ int s_next;
+  __shared__ volatile int s_next;
   if (threadIdx.x == 0) s_next = atomicAdd(queue, 1);
   __syncthreads();
   int t = s_next;
-  while (t < n) {
-    int nxt = 0;
-    if (threadIdx.x == 0) nxt = atomicAdd(queue, 1);
-    const int4 e = tiles[t];
-    const GProblem& p = probs[e.x];
-    const bool vec_store = ((p.ldc & 3) == 0) && ((reinterpret_cast<uintptr_t>(p.C) & 15) == 0);
-    ffma_tile<BM, BN, BK, WM, WN, STAGES, VEC, PAIR>(p.A, p.lda, p.B, p.ldb, p.M, p.N, 0, p.K,
-                                                     e.y, e.z, p.C, p.ldc, vec_store, smem);
-    __syncthreads();  // the tile's last reads of the ring and of s_next are done
-    if (threadIdx.x == 0) s_next = nxt;
-    __syncthreads();
-    t = s_next;
+  if (threadIdx.x >= S::kCompute) {
+    ffma_regs_dec<S::kProducerRegs>();
+    while (t < n) {
+      const int4 e = tiles[t];
+      const GProblem& p = probs[e.x];
+      ffma_produce<S, BM, BN, BK, STAGES, VEC, false, false>(p.A, p.lda, p.B, p.ldb, p.M, p.N, 0,
+                                                             p.K, e.y, e.z, smem);
+      ffma_bar_sync<S::kThreads>(0);
+      ffma_bar_sync<S::kThreads>(0);
+      t = s_next;
+    }
+  } else {
+    ffma_regs_inc<S::kComputeRegs>();
+    while (t < n) {
+      int nxt = 0;
+      if (threadIdx.x == 0) nxt = atomicAdd(queue, 1);
+      const int4 e = tiles[t];
+      const GProblem& p = probs[e.x];
+      const bool vec_store = ((p.ldc & 3) == 0) && ((reinterpret_cast<uintptr_t>(p.C) & 15) == 0);
+      ffma_compute<S, BM, BN, BK, WM, WN, STAGES, PAIR, false, false>(p.M, p.N, 0, p.K, e.y, e.z,
+                                                                      p.C, p.ldc, vec_store, smem);
+      ffma_bar_sync<S::kThreads>(0);
+      if (threadIdx.x == 0) s_next = nxt;
+      ffma_bar_sync<S::kThreads>(0);
+      t = s_next;
+    }
   }
 }
 
@@ -691,23 +709,25 @@ struct GFfmaEntry {
   int smem, threads, per_sm;
   const void* kv;
   const void* ks;
+  bool (*regs_ok)(const void*, int*);
 };
 template <int BM, int BN, int BK, int WM, int WN, int ST, bool PAIR>
 static GFfmaEntry gffma_entry() {
   using S = FfmaShape<BM, BN, BK, WM, WN, ST>;
-  return {S::kSmemBytes, S::kThreads, S::kMinBlocks,
+  return {S::smem_bytes(false, false), S::kThreads, S::kMinBlocks,
           reinterpret_cast<const void*>(&ffma_grouped_kernel<BM, BN, BK, WM, WN, ST, true, PAIR>),
-          reinterpret_cast<const void*>(&ffma_grouped_kernel<BM, BN, BK, WM, WN, ST, false, PAIR>)};
+          reinterpret_cast<const void*>(&ffma_grouped_kernel<BM, BN, BK, WM, WN, ST, false, PAIR>),
+          &ffma_regs_ok<S>};
 }
 static GFfmaEntry gffma_table(int idx) {
   switch (idx) {
     case 0: return gffma_entry<128, 128, 16, 64, 64, 4, true>();
     case 1: return gffma_entry<128, 256, 16, 64, 64, 4, true>();
-    case 2: return gffma_entry<64, 64, 16, 32, 32, 4, true>();
+    case 2: return gffma_entry<64, 64, 16, 32, 32, 6, true>();
     case 3: return gffma_entry<128, 64, 16, 64, 32, 4, true>();
     case 4: return gffma_entry<128, 256, 32, 64, 64, 3, true>();
     case 5: return gffma_entry<256, 128, 16, 64, 64, 4, true>();
-    case 6: return gffma_entry<128, 128, 32, 64, 64, 3, true>();
+    case 6: return gffma_entry<128, 128, 32, 64, 64, 2, true>();
     case 7: return gffma_entry<128, 128, 16, 64, 64, 4, false>();
     default: return gffma_entry<128, 128, 16, 64, 32, 4, true>();
   }
@@ -740,6 +760,7 @@ static const GTcEntry kGTcInline[] = {HBSG_TC_TILE_LIST(HBSG_GTCI_ENTRY)};
 static uint64_t g_tci_masks[sizeof(kGTcInline) / sizeof(kGTcInline[0])][2];
 
 static uint64_t g_ffma_masks[9][2];
+static int g_ffma_regs[9][2];
 static uint64_t g_tc_masks[sizeof(kGTc) / sizeof(kGTc[0])][2];
 
 struct GFusedEntry {
@@ -788,6 +809,8 @@ static cudaError_t grouped_launch(const GroupedPlan& pl, cudaStream_t st) {
     const void* k = pl.vec ? e.kv : e.ks;
     if (!set_smem_once(k, e.smem, &g_ffma_masks[pl.ffma_tile][pl.vec ? 0 : 1]))
       return cudaErrorInvalidValue;
+    if (!e.regs_ok(k, &g_ffma_regs[pl.ffma_tile][pl.vec ? 0 : 1]))
+      return cudaErrorInvalidConfiguration;
     int n = (int)L.num_tiles;
     int* queue = reinterpret_cast<int*>(pl.ws + L.queue_off);
     cudaError_t qe = cudaMemsetAsync(queue, 0, sizeof(int), st);

@@ -27,7 +27,7 @@ struct FfmaParams {
 
 int ffma_num_tiles();
 bool ffma_tile_info(int idx, hbsg_tile_info* out);
-int ffma_pick_tile(int M, int N, int K, int batch, int num_sms);
+int ffma_pick_tile(int M, int N, int K, int batch, int num_sms, bool trans);
 size_t ffma_workspace_bytes(int M, int N, int batch, int splits);
 cudaError_t ffma_launch(int tile_idx, FfmaParams p, int batch, int sms, cudaStream_t st,
                         int ta = 0, int tb = 0);
