@@ -317,14 +317,14 @@ static int gemm_dispatch(int trans_a, int trans_b, int M, int N, int K, const fl
     for (int b = 0; b < batch; ++b) {
       const float* Ab = A + b * strideA;
       const float* Bb = B + b * strideB;
-      cudaError_t e = cudaSuccess;
-      if (scaled && !(flags & HBSG_FLAG_PRESPLIT_A)) e = maxabs_rows(Ab, lda, M, K, rowmax, st);
-      if (e == cudaSuccess && !(flags & HBSG_FLAG_PRESPLIT_B)) {
-        if (ts)  // B's parts (and the scaled forms' column maxima)
-          e = split_operand_b(Bb, ldb, K, N, L.Kp, P, scaled, Bp, colmax, sms, st);
-        else if (scaled)
-          e = maxabs_cols(Bb, ldb, K, N, colmax, st);
-      }
+      // A's maxima, B's parts (A-in-TMEM tiles) and column maxima
+      SplitOperand ops[2];
+      int n_ops = 0;
+      if (scaled && !(flags & HBSG_FLAG_PRESPLIT_A))
+        ops[n_ops++] = {Ab, lda, M, K, L.Kp, false, nullptr, rowmax};
+      if (!(flags & HBSG_FLAG_PRESPLIT_B))
+        ops[n_ops++] = {Bb, ldb, N, K, L.Kp, true, ts ? Bp : nullptr, colmax};
+      cudaError_t e = split_operands(ops, n_ops, P, scaled, st);
       if (e != cudaSuccess) return status_from(e);
       if (flags & HBSG_FLAG_SPLIT_ONLY) continue;
       FusedParams fp{};
@@ -353,17 +353,14 @@ static int gemm_dispatch(int trans_a, int trans_b, int M, int N, int K, const fl
     const float* Ab = A + b * strideA;
     const float* Bb = B + b * strideB;
     float* Cb = C + b * strideC;
-    cudaError_t e = cudaSuccess;
-    if (!(flags & HBSG_FLAG_PRESPLIT_A)) {
-      e = trans_a ? split_operand_b(Ab, lda, K, M, L.Kp, P, scaled, Ap, rowmax, sms, st)
-                  : split_operand_a(Ab, lda, M, K, L.Kp, P, scaled, Ap, rowmax, sms, st);
-      if (e != cudaSuccess) return status_from(e);
-    }
-    if (!(flags & HBSG_FLAG_PRESPLIT_B)) {
-      e = trans_b ? split_operand_a(Bb, ldb, N, K, L.Kp, P, scaled, Bp, colmax, sms, st)
-                  : split_operand_b(Bb, ldb, K, N, L.Kp, P, scaled, Bp, colmax, sms, st);
-      if (e != cudaSuccess) return status_from(e);
-    }
+    SplitOperand ops[2];
+    int n_ops = 0;
+    if (!(flags & HBSG_FLAG_PRESPLIT_A))
+      ops[n_ops++] = {Ab, lda, M, K, L.Kp, trans_a != 0, Ap, rowmax};
+    if (!(flags & HBSG_FLAG_PRESPLIT_B))
+      ops[n_ops++] = {Bb, ldb, N, K, L.Kp, trans_b == 0, Bp, colmax};
+    cudaError_t e = split_operands(ops, n_ops, P, scaled, st);
+    if (e != cudaSuccess) return status_from(e);
     if (flags & HBSG_FLAG_SPLIT_ONLY) continue;
     e = tc_launch(tc, Ap, Bp, M, N, K, L.Kp, Cb, ldc, rowmax, colmax, raster, chunk, sms, 0, 0, st,
                   splits, reinterpret_cast<float*>(w + L.total));

@@ -263,8 +263,8 @@ struct GTilesInline : GTiles {
     const int r = d.r0 + lane;
     const int rows = d.isA ? c.M : c.N;
     if (r >= rows) return;
-    int e = 0;
-    if constexpr (SCALED) e = exp_from_maxbits(d.isA ? c.rowmax[r] : c.colmax[r]);
+    const SplitScale sc =
+        split_scale(SCALED ? exp_from_maxbits(d.isA ? c.rowmax[r] : c.colmax[r]) : 0);
     const long plane = (long)rows * c.Kp;
     __nv_bfloat16* dst = (d.isA ? c.Ap : c.Bp) + (long)r * c.Kp + d.k0;
 #pragma unroll
@@ -273,7 +273,7 @@ struct GTilesInline : GTiles {
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
         __nv_bfloat16 o[3];
-        split_value<P>(v[8 * gi + i], e, o);
+        split_value<P, SCALED>(v[8 * gi + i], sc, o);
 #pragma unroll
         for (int q = 0; q < P; ++q) parts[q][i] = o[q];
       }
@@ -422,30 +422,10 @@ __global__ void __launch_bounds__(256) gsplit_a_kernel(const GProblem* __restric
     const long unit = (long)j.y + u;
     const int m = (int)(unit / upr);
     const int k0 = (int)(unit - (long)m * upr) * 8;
-    const int e = SCALED ? exp_from_maxbits(p.rowmax[m]) : 0;
-    const float* src = p.A + (long)m * p.lda + k0;
+    const SplitScale sc = split_scale(SCALED ? exp_from_maxbits(p.rowmax[m]) : 0);
     float v[8];
-    if (k0 + 8 <= p.K && ((reinterpret_cast<uintptr_t>(src) & 15) == 0)) {
-      const float4 x0 = *reinterpret_cast<const float4*>(src);
-      const float4 x1 = *reinterpret_cast<const float4*>(src + 4);
-      v[0] = x0.x; v[1] = x0.y; v[2] = x0.z; v[3] = x0.w;
-      v[4] = x1.x; v[5] = x1.y; v[6] = x1.z; v[7] = x1.w;
-    } else {
-#pragma unroll
-      for (int i = 0; i < 8; ++i) v[i] = (k0 + i < p.K) ? src[i] : 0.0f;
-    }
-    __align__(16) __nv_bfloat16 parts[P][8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      __nv_bfloat16 o[3];
-      split_value<P>(v[i], e, o);
-#pragma unroll
-      for (int q = 0; q < P; ++q) parts[q][i] = o[q];
-    }
-    __nv_bfloat16* dst = Ap + (long)m * p.Kp + k0;
-#pragma unroll
-    for (int q = 0; q < P; ++q)
-      *reinterpret_cast<uint4*>(dst + q * plane) = *reinterpret_cast<const uint4*>(parts[q]);
+    split_a_load(p.A + (long)m * p.lda + k0, k0, p.K, v);
+    split_a_store<P, SCALED>(v, sc, Ap + (long)m * p.Kp + k0, plane);
   }
 }
 

@@ -33,10 +33,19 @@ cudaError_t ffma_launch(int tile_idx, FfmaParams p, int batch, int sms, cudaStre
                         int ta = 0, int tb = 0);
 
 // ---- split-BF16 family ----------------------------------------------------------
-cudaError_t split_operand_a(const float* A, long lda, int M, int K, int Kp, int parts, bool scaled,
-                            void* Ap, uint32_t* rowmax, int sms, cudaStream_t st);
-cudaError_t split_operand_b(const float* B, long ldb, int K, int N, int Kp, int parts, bool scaled,
-                            void* Bp, uint32_t* colmax, int sms, cudaStream_t st);
+// One operand of the split pass: n output rows of K elements, either stored
+// so (row stride ld) or, with `columns`, as a K x n matrix. parts: [P][n][Kp]
+// BF16 (null: only the maxima); mx: n maxima, written by the scaled forms.
+struct SplitOperand {
+  const float* X;
+  long ld;
+  int n, K, Kp;
+  bool columns;
+  void* parts;
+  uint32_t* mx;
+};
+cudaError_t split_operands(const SplitOperand* ops, int n, int parts, bool scaled,
+                           cudaStream_t st);
 int tc_num_tiles();
 bool tc_tile_info(int idx, hbsg_tile_info* out);
 int tc_tile_parts(int idx);
@@ -110,10 +119,6 @@ bool tc_make_f32_map(void* map, const void* base, int inner, int outer, long ld,
 // K slices of the automatic schedule for `tiles` output tiles on `slots`
 // concurrent work slots (requested > 0 overrides); shared by both families.
 int tc_slices(long tiles, int K, int slots, int requested, int* kt_per_split);
-// Row / column maxima of |x| (FP32 bit patterns) for the scaled forms.
-cudaError_t maxabs_rows(const float* A, long lda, int M, int K, uint32_t* rowmax, cudaStream_t st);
-cudaError_t maxabs_cols(const float* B, long ldb, int K, int N, uint32_t* colmax, cudaStream_t st);
-
 // Workspace of one hbsg_gemm call on these operands (their alignment decides
 // whether a fused-split schedule may run).
 size_t gemm_workspace_exact(int trans_a, int trans_b, int m, int n, int k, const float* a,

@@ -14,148 +14,230 @@
 // FP32 bit patterns (non-negative floats order like their bit patterns, so an
 // integer atomicMax is an exact, order-independent max), then derive
 // e = frexp exponent of that max: the row's largest |x'| lies in [0.5, 1).
+//
+// Bound by HBM (4 bytes read, 2 P written per element) once the operands are
+// large, by launches and latency below that, so both operands share a launch:
+// each is either row-major along k (A, transposed B: "rows") or k x n (B,
+// transposed A: "columns", transposed through shared memory). Unscaled forms
+// take one launch. Scaled forms take two: the first finishes rows (one CTA
+// reads a row for its maximum and again, from the cache, for the split) and
+// reduces the column maxima, the second splits the columns. 3001 x 2503 x
+// 3607 in the scaled 3-product form: 71 -> 48 us of split
+// work, 4 launches and a memset before. At 8192^3 the passes run at 6.1 TB/s.
 #include "internal.h"
 #include "split_kernel.cuh"
 
 namespace hbsg {
 
-// max|A[m][k]| over k per row, one warp per row.
-__global__ void row_maxabs_kernel(const float* __restrict__ A, long lda, int M, int K,
-                                  uint32_t* __restrict__ out) {
-  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (warp >= M) return;
-  const float* row = A + (long)warp * lda;
-  float mx = 0.0f;
-  for (int k = lane; k < K; k += 32) {
-    const float a = fabsf(row[k]);
-    if (isfinite(a)) mx = fmaxf(mx, a);
-  }
+static constexpr int kSplitThreads = 256;
+// Rows up to this long are finished by one CTA each (max and split); longer
+// ones are cut into chunks of this many k for the maximum.
+static constexpr int kRowChunk = 16384;
+static constexpr int kColRows = 64;  // k rows per CTA of the column maxima
+
+// One operand's share of a launch (blocks [first, first + blocks)).
+enum SplitRole { kRowSplit, kRowMaxSplit, kRowMax, kColMax, kColSplit };
+struct SplitJob {
+  const float* X;  // rows: n x K with row stride ld; columns: K x n
+  long ld;
+  __nv_bfloat16* parts;  // [P][n][Kp], null: maxima only
+  uint32_t* mx;          // n maxima (scaled forms)
+  int n, K, Kp;
+  int role;
+  unsigned blocks;
+};
+struct SplitJobs {
+  SplitJob job[2];
+  unsigned first1;  // first block of job[1]
+};
+
+HBSG_DEV float finite_abs(float x) {
+  const float a = fabsf(x);
+  return isfinite(a) ? a : 0.0f;
+}
+
+HBSG_DEV float block_max(float mx, float* red) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-  if (lane == 0) out[warp] = __float_as_uint(mx);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = mx;
+  __syncthreads();
+  mx = red[threadIdx.x & (kSplitThreads / 32 - 1)];
+#pragma unroll
+  for (int o = kSplitThreads / 64; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+  return mx;
 }
 
-// max|B[k][n]| over k per column: threads along n, blocks along k slices.
-__global__ void col_maxabs_kernel(const float* __restrict__ B, long ldb, int K, int N,
-                                  int k_per_block, uint32_t* __restrict__ out) {
-  const int n = blockIdx.x * blockDim.x + threadIdx.x;
-  if (n >= N) return;
-  const int k0 = blockIdx.y * k_per_block;
-  const int k1 = min(K, k0 + k_per_block);
+// max|row[k]| over k in [k0, k1) by the whole CTA.
+HBSG_DEV float row_max(const float* __restrict__ row, int k0, int k1, float* red) {
   float mx = 0.0f;
-  for (int k = k0; k < k1; ++k) {
-    const float b = fabsf(B[(long)k * ldb + n]);
-    if (isfinite(b)) mx = fmaxf(mx, b);
+  if ((reinterpret_cast<uintptr_t>(row + k0) & 15) == 0) {
+    const int k4 = k0 + (k1 - k0) / 4 * 4;
+    for (int k = k0 + 4 * (int)threadIdx.x; k < k4; k += 4 * kSplitThreads) {
+      const float4 v = *reinterpret_cast<const float4*>(row + k);
+      mx = fmaxf(fmaxf(mx, fmaxf(finite_abs(v.x), finite_abs(v.y))),
+                 fmaxf(finite_abs(v.z), finite_abs(v.w)));
+    }
+    k0 = k4;
   }
-  if (mx > 0.0f) atomicMax(out + n, __float_as_uint(mx));
+  for (int k = k0 + (int)threadIdx.x; k < k1; k += kSplitThreads) mx = fmaxf(mx, finite_abs(row[k]));
+  return block_max(mx, red);
 }
 
-// A (M x K, row stride lda) -> Ap[p][m][0..Kp). One thread per 8 consecutive k.
 template <int P, bool SCALED>
-__global__ void split_a_kernel(const float* __restrict__ A, long lda, int M, int K, int Kp,
-                               __nv_bfloat16* __restrict__ Ap, const uint32_t* __restrict__ rowmax) {
-  const long groups_per_row = Kp / 8;
-  const long total = (long)M * groups_per_row;
-  const long plane = (long)M * Kp;
-  for (long g = blockIdx.x * (long)blockDim.x + threadIdx.x; g < total;
-       g += (long)gridDim.x * blockDim.x) {
-    const int m = (int)(g / groups_per_row);
-    const int k0 = (int)(g - (long)m * groups_per_row) * 8;
-    const int e = SCALED ? exp_from_maxbits(rowmax[m]) : 0;
-    const float* src = A + (long)m * lda + k0;
-    float v[8];
-    if (k0 + 8 <= K && ((reinterpret_cast<uintptr_t>(src) & 15) == 0)) {
-      const float4 x0 = *reinterpret_cast<const float4*>(src);
-      const float4 x1 = *reinterpret_cast<const float4*>(src + 4);
-      v[0] = x0.x; v[1] = x0.y; v[2] = x0.z; v[3] = x0.w;
-      v[4] = x1.x; v[5] = x1.y; v[6] = x1.z; v[7] = x1.w;
-    } else {
+HBSG_DEV void split_job(const SplitJob& j, unsigned block, float (*tile)[65]) {
+  switch (j.role) {
+    case kRowSplit: {  // 8 consecutive k per thread, 4 units a block apart
+      const unsigned upr = (unsigned)j.Kp / 8;
+      const long total = (long)j.n * upr;
+      const long plane = (long)j.n * j.Kp;
 #pragma unroll
-      for (int i = 0; i < 8; ++i) v[i] = (k0 + i < K) ? src[i] : 0.0f;
+      for (int u = 0; u < 4; ++u) {
+        const long g = ((long)block * 4 + u) * kSplitThreads + threadIdx.x;
+        if (g >= total) return;
+        const long m = total <= 0xffffffffL ? (long)((unsigned)g / upr) : g / upr;
+        const int k0 = (int)(g - m * upr) * 8;
+        const SplitScale sc = split_scale(SCALED ? exp_from_maxbits(j.mx[m]) : 0);
+        float v[8];
+        split_a_load(j.X + m * j.ld + k0, k0, j.K, v);
+        split_a_store<P, SCALED>(v, sc, j.parts + m * j.Kp + k0, plane);
+      }
+      break;
     }
-    __align__(16) __nv_bfloat16 parts[P][8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      __nv_bfloat16 o[3];
-      split_value<P>(v[i], e, o);
-#pragma unroll
-      for (int p = 0; p < P; ++p) parts[p][i] = o[p];
+    case kRowMaxSplit: {  // one row: its maximum, then its split
+      const float* row = j.X + (long)block * j.ld;
+      const float mx = row_max(row, 0, j.K, tile[0]);
+      if (threadIdx.x == 0) j.mx[block] = __float_as_uint(mx);
+      if (!j.parts) return;
+      const SplitScale sc = split_scale(exp_from_maxbits(__float_as_uint(mx)));
+      const long plane = (long)j.n * j.Kp;
+      for (int k0 = 8 * (int)threadIdx.x; k0 < j.Kp; k0 += 8 * kSplitThreads) {
+        float v[8];
+        split_a_load(row + k0, k0, j.K, v);
+        split_a_store<P, SCALED>(v, sc, j.parts + (long)block * j.Kp + k0, plane);
+      }
+      break;
     }
-    __nv_bfloat16* dst = Ap + (long)m * Kp + k0;
+    case kRowMax: {  // one chunk of a long row into its (zeroed) maximum
+      const int chunks = (j.K + kRowChunk - 1) / kRowChunk;
+      const int r = (int)(block / (unsigned)chunks);
+      const int k0 = (int)(block % (unsigned)chunks) * kRowChunk;
+      const float mx = row_max(j.X + (long)r * j.ld, k0, min(j.K, k0 + kRowChunk), tile[0]);
+      if (threadIdx.x == 0 && mx > 0.0f) atomicMax(j.mx + r, __float_as_uint(mx));
+      break;
+    }
+    case kColMax: {  // 256 columns x kColRows k into the (zeroed) maxima
+      const unsigned nb = ((unsigned)j.n + kSplitThreads - 1) / kSplitThreads;
+      const int n = (int)(block % nb) * kSplitThreads + (int)threadIdx.x;
+      const int k0 = (int)(block / nb) * kColRows;
+      if (n >= j.n) return;
+      const int k1 = min(j.K, k0 + kColRows);
+      const float* p = j.X + (long)k0 * j.ld + n;
+      float mx = 0.0f;
+      int k = k0;
+      for (; k + 8 <= k1; k += 8, p += 8 * j.ld) {
+        float v[8];
 #pragma unroll
-    for (int p = 0; p < P; ++p)
-      *reinterpret_cast<uint4*>(dst + p * plane) = *reinterpret_cast<const uint4*>(parts[p]);
+        for (int i = 0; i < 8; ++i) v[i] = p[i * j.ld];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) mx = fmaxf(mx, finite_abs(v[i]));
+      }
+      for (; k < k1; ++k, p += j.ld) mx = fmaxf(mx, finite_abs(*p));
+      if (mx > 0.0f) atomicMax(j.mx + n, __float_as_uint(mx));
+      break;
+    }
+    default: {  // kColSplit: one 64 x 64 block, transposed
+      const unsigned nb = ((unsigned)j.n + 63) / 64;
+      const int n0 = (int)(block % nb) * 64, k0 = (int)(block / nb) * 64;
+      float v[16];
+      split_b_load(j.X, j.ld, j.K, j.n, k0, n0, v);
+      split_b_to_tile(v, tile);
+      __syncthreads();
+      split_b_from_tile<P, SCALED>(j.n, j.Kp, j.parts, j.mx, k0, n0, tile);
+    }
   }
 }
 
-// B (K x N, row stride ldb) -> Bp[p][n][0..Kp) through 64 x 64 shared tiles.
 template <int P, bool SCALED>
-__global__ void __launch_bounds__(256) split_b_kernel(const float* __restrict__ B, long ldb, int K,
-                                                      int N, int Kp, __nv_bfloat16* __restrict__ Bp,
-                                                      const uint32_t* __restrict__ colmax) {
+__global__ void __launch_bounds__(kSplitThreads) split_kernel(const __grid_constant__ SplitJobs jobs) {
   __shared__ float tile[64][65];
-  split_b_block<P, SCALED>(B, ldb, K, N, Kp, Bp, colmax, blockIdx.y * 64, blockIdx.x * 64, tile);
+  if (blockIdx.x < jobs.first1) split_job<P, SCALED>(jobs.job[0], blockIdx.x, tile);
+  else split_job<P, SCALED>(jobs.job[1], blockIdx.x - jobs.first1, tile);
 }
 
-cudaError_t maxabs_rows(const float* A, long lda, int M, int K, uint32_t* rowmax, cudaStream_t st) {
-  if (M > 0) row_maxabs_kernel<<<(M + 7) / 8, 256, 0, st>>>(A, lda, M, K, rowmax);
-  return cudaGetLastError();
-}
-
-cudaError_t maxabs_cols(const float* B, long ldb, int K, int N, uint32_t* colmax, cudaStream_t st) {
-  cudaError_t e = cudaMemsetAsync(colmax, 0, sizeof(uint32_t) * N, st);
-  if (e != cudaSuccess) return e;
-  const int kpb = 256;
-  dim3 g((N + 255) / 256, (K + kpb - 1) / kpb);
-  if (K > 0 && N > 0) col_maxabs_kernel<<<g, 256, 0, st>>>(B, ldb, K, N, kpb, colmax);
-  return cudaGetLastError();
-}
-
-static int grid_for(long work, int per_block, int sms) {
-  long b = (work + per_block - 1) / per_block;
-  const long cap = (long)sms * 8;
-  return (int)(b < cap ? (b > 0 ? b : 1) : cap);
-}
-
-cudaError_t split_operand_a(const float* A, long lda, int M, int K, int Kp, int parts, bool scaled,
-                            void* Ap, uint32_t* rowmax, int sms, cudaStream_t st) {
-  if (scaled) {
-    row_maxabs_kernel<<<(M + 7) / 8, 256, 0, st>>>(A, lda, M, K, rowmax);
+static long blocks_of(const SplitJob& j) {
+  auto cdiv = [](long a, long b) { return (a + b - 1) / b; };
+  switch (j.role) {
+    case kRowSplit: return cdiv((long)j.n * (j.Kp / 8), 4 * kSplitThreads);
+    case kRowMaxSplit: return j.n;
+    case kRowMax: return (long)j.n * cdiv(j.K, kRowChunk);
+    case kColMax: return cdiv(j.n, kSplitThreads) * cdiv(j.K, kColRows);
+    default: return cdiv(j.n, 64) * cdiv(j.Kp, 64);
   }
-  const long work = (long)M * (Kp / 8);
-  const int grid = grid_for(work, 256, sms);
-  auto* ap = static_cast<__nv_bfloat16*>(Ap);
-  if (parts == 3) {
-    if (scaled) split_a_kernel<3, true><<<grid, 256, 0, st>>>(A, lda, M, K, Kp, ap, rowmax);
-    else split_a_kernel<3, false><<<grid, 256, 0, st>>>(A, lda, M, K, Kp, ap, rowmax);
-  } else {
-    if (scaled) split_a_kernel<2, true><<<grid, 256, 0, st>>>(A, lda, M, K, Kp, ap, rowmax);
-    else split_a_kernel<2, false><<<grid, 256, 0, st>>>(A, lda, M, K, Kp, ap, rowmax);
-  }
-  return cudaGetLastError();
 }
 
-cudaError_t split_operand_b(const float* B, long ldb, int K, int N, int Kp, int parts, bool scaled,
-                            void* Bp, uint32_t* colmax, int sms, cudaStream_t st) {
-  if (scaled) {
-    cudaError_t e = cudaMemsetAsync(colmax, 0, sizeof(uint32_t) * N, st);
-    if (e != cudaSuccess) return e;
-    const int kpb = 256;
-    dim3 g((N + 255) / 256, (K + kpb - 1) / kpb);
-    if (K > 0) col_maxabs_kernel<<<g, 256, 0, st>>>(B, ldb, K, N, kpb, colmax);
+static cudaError_t launch_jobs(SplitJob* job, int n, int parts, bool scaled, cudaStream_t st) {
+  // grids are one-dimensional: at most 2^31 - 1 blocks, each launch takes as
+  // many jobs as fit (one operand alone always does: its elements are
+  // addressable by 32-bit row and k)
+  SplitJobs jobs{};
+  long total = 0;
+  int taken = 0;
+  auto flush = [&]() -> cudaError_t {
+    if (total == 0) return cudaSuccess;
+    const unsigned grid = (unsigned)total;
+    if (parts == 3) {
+      if (scaled) split_kernel<3, true><<<grid, kSplitThreads, 0, st>>>(jobs);
+      else split_kernel<3, false><<<grid, kSplitThreads, 0, st>>>(jobs);
+    } else {
+      if (scaled) split_kernel<2, true><<<grid, kSplitThreads, 0, st>>>(jobs);
+      else split_kernel<2, false><<<grid, kSplitThreads, 0, st>>>(jobs);
+    }
+    total = 0;
+    taken = 0;
+    return cudaGetLastError();
+  };
+  for (int i = 0; i < n; ++i) {
+    const long b = blocks_of(job[i]);
+    if (b <= 0) continue;
+    if (b > 0x7fffffffL) return cudaErrorInvalidConfiguration;
+    if (total + b > 0x7fffffffL) {
+      const cudaError_t e = flush();
+      if (e != cudaSuccess) return e;
+    }
+    job[i].blocks = (unsigned)b;
+    jobs.job[taken] = job[i];
+    total += b;
+    if (taken == 0) jobs.first1 = (unsigned)b;
+    ++taken;
   }
-  dim3 grid((N + 63) / 64, (Kp + 63) / 64);
-  auto* bp = static_cast<__nv_bfloat16*>(Bp);
-  (void)sms;
-  if (parts == 3) {
-    if (scaled) split_b_kernel<3, true><<<grid, 256, 0, st>>>(B, ldb, K, N, Kp, bp, colmax);
-    else split_b_kernel<3, false><<<grid, 256, 0, st>>>(B, ldb, K, N, Kp, bp, colmax);
-  } else {
-    if (scaled) split_b_kernel<2, true><<<grid, 256, 0, st>>>(B, ldb, K, N, Kp, bp, colmax);
-    else split_b_kernel<2, false><<<grid, 256, 0, st>>>(B, ldb, K, N, Kp, bp, colmax);
+  return flush();
+}
+
+cudaError_t split_operands(const SplitOperand* ops, int n, int parts, bool scaled,
+                           cudaStream_t st) {
+  SplitJob first[2], second[2];
+  int n1 = 0, n2 = 0;
+  for (int i = 0; i < n; ++i) {
+    const SplitOperand& o = ops[i];
+    if (o.n <= 0 || (!o.parts && !scaled)) continue;
+    SplitJob j{o.X, o.ld, static_cast<__nv_bfloat16*>(o.parts), o.mx, o.n, o.K, o.Kp, 0, 0};
+    if (!scaled) {
+      j.role = o.columns ? kColSplit : kRowSplit;
+      first[n1++] = j;
+    } else if (!o.columns && o.K <= kRowChunk) {
+      j.role = kRowMaxSplit;
+      first[n1++] = j;
+    } else {
+      const cudaError_t e = cudaMemsetAsync(o.mx, 0, sizeof(uint32_t) * (size_t)o.n, st);
+      if (e != cudaSuccess) return e;
+      j.role = o.columns ? kColMax : kRowMax;
+      if (o.K > 0) first[n1++] = j;
+      j.role = o.columns ? kColSplit : kRowSplit;
+      if (o.parts) second[n2++] = j;
+    }
   }
-  return cudaGetLastError();
+  const cudaError_t e = launch_jobs(first, n1, parts, scaled, st);
+  return e != cudaSuccess ? e : launch_jobs(second, n2, parts, scaled, st);
 }
 
 }  // namespace hbsg

@@ -223,10 +223,9 @@ HBSG_DEV void tmem_ld16(uint32_t taddr, float* v) {
 template <int P, bool SCALED>
 HBSG_DEV void split8(float (&x)[8], int e, uint4 (&out)[P]) {
   if constexpr (SCALED) {
-    if (e != 0) {
+    const SplitScale sc = split_scale(e);
 #pragma unroll
-      for (int i = 0; i < 8; ++i) x[i] = ldexpf(x[i], -e);
-    }
+    for (int i = 0; i < 8; ++i) x[i] = apply_scale(x[i], sc);
   }
   uint32_t h[4], m[4], l[4];
 #pragma unroll
