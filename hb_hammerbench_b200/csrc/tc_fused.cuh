@@ -373,7 +373,7 @@ __device__ __forceinline__ void tc_fused_body(const Tiles& tiles, const TcRun& r
   if (warp == 0) {
     // ---------------- MMA issuer (leader CTA only) ----------------
     // The whole warp runs the loop converged and one elected lane issues
-    // (tc_mma_elect); a wait passes only when it passed on every lane.
+    // (tc_issue_ktile); a wait passes only when it passed on every lane.
     if (leader) {
       // full-width MMAs: each CTA holds a fixed half of the BN columns, so the
       // instruction's N cannot be trimmed (padding columns are zeros)
@@ -387,38 +387,33 @@ __device__ __forceinline__ void tc_fused_body(const Tiles& tiles, const TcRun& r
         int kt = 0;
         for (int c = 0; c < nchunks && ok; ++c, ++ch) {
           const int buf = ch & 1;
-          if (!__all_sync(0xffffffffu,
-                          wait_bounded(&tempty[buf], ((ch >> 1) & 1) ^ 1, abort_flag, lim))) {
-            ok = false;
-            break;
-          }
-          tc_fence_after();
           const uint32_t d = tmem_base + buf * BN;
           const int kend = min(KT, kt + run.chunk_ktiles);
-          bool first = true;
+          uint32_t accumulate = 0;  // 0: the chunk's first k-tile, which also needs the buffer
           for (; kt < kend; ++kt, ++it) {
             const int s = it % STAGES;
-            if (!__all_sync(0xffffffffu, wait_bounded_cluster(&full[s], (it / STAGES) & 1,
-                                                              abort_flag, lim))) {
-              ok = false;
-              break;
+            const uint32_t pf = (it / STAGES) & 1, pt = ((ch >> 1) & 1) ^ 1;
+            bool ready = mbar_try_wait_cluster(&full[s], pf);
+            if (!accumulate) ready = mbar_try_wait(&tempty[buf], pt) && ready;
+            if (!__all_sync(0xffffffffu, ready)) {
+              ready = (accumulate || wait_bounded(&tempty[buf], pt, abort_flag, lim)) &&
+                      wait_bounded_cluster(&full[s], pf, abort_flag, lim);
+              if (!__all_sync(0xffffffffu, ready)) {
+                ok = false;
+                break;
+              }
             }
             tc_fence_after();
             const uint32_t sa = base + s * S::kStageBytes;
-            const uint32_t sb = sa + P * S::kABytes;
-#pragma unroll
-            for (int ks = 0; ks < kBK / 16; ++ks) {
-#pragma unroll
-              for (int q = 0; q < Products<P>::n; ++q) {
-                const uint64_t ad = sw64_desc(sa + Products<P>::a(q) * S::kABytes + ks * 32);
-                const uint64_t bd = sw64_desc(sb + Products<P>::b(q) * S::kBBytes + ks * 32);
-                tc_mma_pair_elect(d, ad, bd, idesc, first ? 0u : 1u);
-                first = false;
-              }
+            if (tc_elect()) {
+              tc_issue_ktile<P, S::kABytes, S::kBBytes, true>(d, sa, sa + P * S::kABytes, idesc,
+                                                              accumulate);
+              tc_commit<true>(&empty[s]);
+              if (kt + 1 == kend) tc_commit<true>(&tfull[buf]);
             }
-            tc_commit_pair_elect(&empty[s]);
+            __syncwarp();
+            accumulate = 1;
           }
-          if (ok) tc_commit_pair_elect(&tfull[buf]);
         }
       }
     }
@@ -603,8 +598,7 @@ __device__ __forceinline__ void tc_fused_body(const Tiles& tiles, const TcRun& r
         for (int j = 0; j < COLS / 16; ++j) {
           float vv[16];
           tmem_ld16(taddr + 16 * j, vv);
-#pragma unroll
-          for (int i = 0; i < 16; ++i) sum[16 * j + i] += vv[i];
+          add_drained<16>(sum + 16 * j, vv);
         }
         tc_fence_before();
         __syncwarp();

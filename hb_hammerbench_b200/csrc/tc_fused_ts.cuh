@@ -21,9 +21,9 @@
 // read it. The two operands therefore have rings of their own, each with its
 // own loader thread, so the A loads run ahead of the MMAs in flight. The MMA
 // issuer is a whole converged warp with one elected lane issuing (a loop on a
-// single lane spent ~70 cycles per N = 64 MMA issued, measured per role, about
-// twice the tensor core's time for one: 87 against 122 TFLOP/s for the
-// 6-product 65536 x 64 x 4096).
+// single lane, its waits and commits included, spent ~70 cycles per N = 64 MMA
+// issued, about twice the tensor core's time for one: 87 against 122 TFLOP/s
+// for the 6-product 65536 x 64 x 4096).
 //
 // Layouts:
 //   - shared memory: the FP32 A staging ring (SA stages of 128 rows x 32 k,
@@ -106,16 +106,14 @@ HBSG_DEV void tmem_st8(uint32_t taddr, const uint32_t (&r)[8]) {
 
 HBSG_DEV void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory"); }
 
-// D (TMEM) (+)= A (TMEM, K-major) x B (shared memory descriptor), M = 128,
-// called by a whole converged warp: elect.sync picks the one lane that
-// issues it.
-HBSG_DEV void tc_mma_ts_elect(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc,
-                              uint32_t accumulate) {
+// D (TMEM) (+)= A (TMEM, K-major) x B (shared memory descriptor), M = 128, by
+// the elected lane of the issuing warp (see tc_issue_ktile).
+HBSG_DEV void tc_mma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc,
+                        uint32_t accumulate) {
   asm volatile(
-      "{\n\t.reg .pred p, e;\n\t.reg .b32 l;\n\t"
-      "elect.sync l|e, 0xffffffff;\n\t"
+      "{\n\t.reg .pred p;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
-      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}\n" ::"r"(d_tmem),
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}\n" ::"r"(d_tmem),
       "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate));
 }
 
@@ -217,12 +215,12 @@ __device__ __forceinline__ void tc_fused_ts_body(const Tiles& tiles, const TcRun
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
-    // The loop runs converged on all 32 lanes of the warp, so its operands
-    // (TMEM addresses, descriptors) are warp-uniform, and one elected lane
-    // issues each MMA and commit (a loop on a single lane measured ~70
-    // cycles per N = 64 MMA issued, about twice the tensor core's time for
-    // one). Every lane takes the bounded waits; a wait counts as passed only
-    // when it passed on all lanes.
+    // The loop runs converged on all 32 lanes of the warp and one elected lane
+    // issues (see tc_issue_ktile). Every lane takes the bounded waits; a wait
+    // counts as passed only when it passed on all lanes. Measured per k-tile of
+    // 65536 x 64 x 4096 (6 products, cycles by role counters): 381 of MMA issue
+    // (its tensor-core time) but 684 of waits, commits and loop around it, and
+    // the converters waiting for this warp; 848 in all in this form.
     constexpr uint32_t idesc = f16_idesc(kBM, BN);
     uint32_t it = 0, ch = 0;
     bool ok = true;
@@ -233,41 +231,44 @@ __device__ __forceinline__ void tc_fused_ts_body(const Tiles& tiles, const TcRun
       int kt = 0;
       for (int c = 0; c < nchunks && ok; ++c, ++ch) {
         const int buf = ch & 1;
-        if (!__all_sync(0xffffffffu,
-                        wait_bounded(&tempty[buf], ((ch >> 1) & 1) ^ 1, abort_flag, lim))) {
-          ok = false;
-          break;
-        }
-        tc_fence_after();
         const uint32_t d = tmem_base + buf * BN;
         const int kend = min(KT, kt + run.chunk_ktiles);
-        bool first = true;
+        uint32_t accumulate = 0;  // 0: the chunk's first k-tile, which also needs the buffer
         for (; kt < kend; ++kt, ++it) {
           const int sb = it % SB;
           const int j = it % TSTAGES;
-          const bool got = wait_bounded(&bfull[sb], (it / SB) & 1, abort_flag, lim) &&
-                           wait_bounded(&afull[j], (it / TSTAGES) & 1, abort_flag, lim);
-          if (!__all_sync(0xffffffffu, got)) {
-            ok = false;
-            break;
-          }
-          tc_fence_after();
-          const uint32_t bs = base + S::kBRingOff + sb * S::kSBBytes;
-          const uint32_t ta = tmem_base + S::kAColBase + j * S::kACols;
-#pragma unroll
-          for (int ks = 0; ks < kBK / 16; ++ks) {
-#pragma unroll
-            for (int q = 0; q < Products<P>::n; ++q) {
-              const uint64_t bd = sw64_desc(bs + Products<P>::b(q) * S::kBPart + ks * 32);
-              tc_mma_ts_elect(d, ta + Products<P>::a(q) * (kBK / 2) + ks * 8, bd, idesc,
-                              first ? 0u : 1u);
-              first = false;
+          const uint32_t pb = (it / SB) & 1, pa = (it / TSTAGES) & 1, pt = ((ch >> 1) & 1) ^ 1;
+          const bool rb = mbar_try_wait(&bfull[sb], pb);
+          bool ready = mbar_try_wait(&afull[j], pa) && rb;
+          if (!accumulate) ready = mbar_try_wait(&tempty[buf], pt) && ready;
+          if (!__all_sync(0xffffffffu, ready)) {
+            ready = (accumulate || wait_bounded(&tempty[buf], pt, abort_flag, lim)) &&
+                    wait_bounded(&bfull[sb], pb, abort_flag, lim) &&
+                    wait_bounded(&afull[j], pa, abort_flag, lim);
+            if (!__all_sync(0xffffffffu, ready)) {
+              ok = false;
+              break;
             }
           }
-          tc_commit_elect(&bempty[sb]);
-          tc_commit_elect(&aempty[j]);
+          tc_fence_after();
+          const uint32_t ta = tmem_base + S::kAColBase + j * S::kACols;
+          if (tc_elect()) {
+            const uint64_t bd = sw64_desc(base + S::kBRingOff + sb * S::kSBBytes);
+#pragma unroll
+            for (int ks = 0; ks < kBK / 16; ++ks) {
+#pragma unroll
+              for (int q = 0; q < Products<P>::n; ++q)
+                tc_mma_ts(d, ta + Products<P>::a(q) * (kBK / 2) + ks * 8,
+                          bd + ((Products<P>::b(q) * S::kBPart + ks * 32) >> 4), idesc,
+                          ks == 0 && q == 0 ? accumulate : 1u);
+            }
+            tc_commit<false>(&bempty[sb]);
+            tc_commit<false>(&aempty[j]);
+            if (kt + 1 == kend) tc_commit<false>(&tfull[buf]);
+          }
+          __syncwarp();
+          accumulate = 1;
         }
-        if (ok) tc_commit_elect(&tfull[buf]);
       }
     }
   } else if (warp >= 4 && warp < 4 + 4 * kTsAGroups) {
@@ -352,7 +353,7 @@ __device__ __forceinline__ void tc_fused_ts_body(const Tiles& tiles, const TcRun
       for (int c = 0; c < nchunks; ++c, ++ch) {
         const int buf = ch & 1;
         int got = 0;
-        if (lane == 0) got = wait_bounded_sleep(&tfull[buf], (ch >> 1) & 1, abort_flag, lim);
+        if (lane == 0) got = wait_bounded_hint(&tfull[buf], (ch >> 1) & 1, abort_flag, lim);
         got = __shfl_sync(0xffffffffu, got, 0);
         if (!got) {
           ok = false;
@@ -361,11 +362,10 @@ __device__ __forceinline__ void tc_fused_ts_body(const Tiles& tiles, const TcRun
         tc_fence_after();
         const uint32_t taddr = tmem_base + ((uint32_t)(32 * q) << 16) + buf * BN;
 #pragma unroll
-        for (int jj = 0; jj < BN / 16; ++jj) {
-          float vv[16];
-          tmem_ld16(taddr + 16 * jj, vv);
-#pragma unroll
-          for (int i = 0; i < 16; ++i) sum[16 * jj + i] += vv[i];
+        for (int jj = 0; jj < BN / 32; ++jj) {
+          float vv[32];
+          tmem_ld32(taddr + 32 * jj, vv);
+          add_drained<32>(sum + 32 * jj, vv);
         }
         tc_fence_before();
         __syncwarp();

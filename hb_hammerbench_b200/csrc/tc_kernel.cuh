@@ -99,28 +99,59 @@ HBSG_DEV void tma_prefetch_3d(const CUtensorMap* map, int c0, int c1, int c2) {
 HBSG_DEV void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory"); }
 HBSG_DEV void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory"); }
 
-// Issue forms for a whole converged warp: elect.sync picks the one lane that
-// issues, and the loop around them runs on all lanes with warp-uniform
-// operands (TMEM addresses, descriptors). The same loop run inside a branch
-// taken by lane 0 alone measured ~70 cycles per MMA issued, against the ~32
-// an M = 128, N = 64, K = 16 MMA takes on the tensor core.
-HBSG_DEV void tc_mma_elect(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                           uint32_t accumulate) {
+// The MMA issue. The issuer is a whole warp that runs its loop converged; for
+// each k-tile one elected lane (elect.sync: always the same one) issues the
+// k-tile's MMAs and its commits in one branch, from descriptors formed once
+// per k-tile. The issuer shares its scheduler with the epilogue (and
+// converter) warps, so its instructions count: with three busy warps beside
+// it a loop that elected a lane and built two descriptors per MMA took 112
+// cycles for each N = 64 MMA, this form 65 (the tensor core needs 32; alone
+// both reach that). For the same reason the barriers of a k-tile are probed
+// together and voted on once.
+HBSG_DEV bool tc_elect() {
+  uint32_t e;
   asm volatile(
-      "{\n\t.reg .pred p, e;\n\t.reg .b32 l;\n\t"
-      "elect.sync l|e, 0xffffffff;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d_tmem),
-      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate));
+      "{\n\t.reg .pred p;\n\t.reg .b32 l;\n\t"
+      "elect.sync l|p, 0xffffffff;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}\n"
+      : "=r"(e));
+  return e != 0;
 }
 
-HBSG_DEV void tc_commit_elect(uint64_t* bar) {
-  asm volatile(
-      "{\n\t.reg .pred e;\n\t.reg .b32 l;\n\t"
-      "elect.sync l|e, 0xffffffff;\n\t"
-      "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}\n" ::"r"(
-          smem_u32(bar))
-      : "memory");
+// PAIR: the CTA-pair MMA (cta_group::2), and the commit that arrives (once) on
+// the barrier at this offset in both CTAs of the pair when all prior
+// tensor-core work of the issuing thread completes.
+template <bool PAIR>
+HBSG_DEV void tc_mma(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
+                     uint32_t accumulate) {
+  if constexpr (PAIR)
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d_tmem),
+        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate));
+  else
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d_tmem),
+        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate));
+}
+
+template <bool PAIR>
+HBSG_DEV void tc_commit(uint64_t* bar) {
+  if constexpr (PAIR)
+    asm volatile(
+        "{\n\t.reg .b16 m;\n\t"
+        "mov.b16 m, 3;\n\t"
+        "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64"
+        " [%0], m;\n\t}\n" ::"r"(smem_u32(bar))
+        : "memory");
+  else
+    asm volatile(
+        "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(
+            smem_u32(bar))
+        : "memory");
 }
 
 // 32 lanes x 32 columns of 32-bit TMEM into 32 registers per thread.
@@ -177,6 +208,36 @@ static_assert(Products<3>::a(5) == 0 && Products<3>::b(5) == 0, "hi*hi");
 static_assert(Products<2>::a(0) == 0 && Products<2>::b(0) == 1, "hi*mid");
 static_assert(Products<2>::a(1) == 1 && Products<2>::b(1) == 0, "mid*hi");
 static_assert(Products<2>::a(2) == 0 && Products<2>::b(2) == 0, "hi*hi");
+
+// All MMAs of one k-tile whose parts lie at shared addresses sa (P parts of
+// ABYTES) and sb (P parts of BBYTES), by the elected lane. The descriptors'
+// address field counts 16-byte units and never carries (shared memory ends
+// below 2^18).
+template <int P, int ABYTES, int BBYTES, bool PAIR>
+HBSG_DEV void tc_issue_ktile(uint32_t d, uint32_t sa, uint32_t sb, uint32_t idesc,
+                             uint32_t accumulate) {
+  const uint64_t ad = sw64_desc(sa), bd = sw64_desc(sb);
+#pragma unroll
+  for (int ks = 0; ks < kBK / 16; ++ks) {
+#pragma unroll
+    for (int q = 0; q < Products<P>::n; ++q)
+      tc_mma<PAIR>(d, ad + ((Products<P>::a(q) * ABYTES + ks * 32) >> 4),
+                   bd + ((Products<P>::b(q) * BBYTES + ks * 32) >> 4), idesc,
+                   ks == 0 && q == 0 ? accumulate : 1u);
+  }
+}
+
+// One TMEM column block of a drain: sum += v, two lanes per add instruction
+// (the same IEEE additions).
+template <int COLS>
+HBSG_DEV void add_drained(float* sum, const float* v) {
+#pragma unroll
+  for (int i = 0; i < COLS; i += 2) {
+    const float2 r = __fadd2_rn(make_float2(sum[i], sum[i + 1]), make_float2(v[i], v[i + 1]));
+    sum[i] = r.x;
+    sum[i + 1] = r.y;
+  }
+}
 
 template <int P, int BN, int STAGES>
 struct TcShape {
@@ -493,7 +554,7 @@ __device__ __forceinline__ void tc_body(const Tiles& tiles, const TcRun& run) {
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
     // The whole warp runs the loop converged and one elected lane issues
-    // (tc_mma_elect); lane 0 takes the tile queue's entries for the warp, and
+    // (tc_issue_ktile); lane 0 takes the tile queue's entries for the warp, and
     // a wait passes only when it passed on every lane.
     {
       uint32_t it = 0, ch = 0, q = 0;
@@ -535,38 +596,33 @@ __device__ __forceinline__ void tc_body(const Tiles& tiles, const TcRun& run) {
         int kt = 0;
         for (int c = 0; c < nchunks && ok; ++c, ++ch) {
           const int buf = ch & 1;
-          if (!__all_sync(0xffffffffu,
-                          wait_bounded(&tempty[buf], ((ch >> 1) & 1) ^ 1, abort_flag, lim))) {
-            ok = false;
-            break;
-          }
-          tc_fence_after();
           const uint32_t d = tmem_base + buf * BN;
           const int kend = min(KT, kt + run.chunk_ktiles);
-          bool first = true;
+          uint32_t accumulate = 0;  // 0: the chunk's first k-tile, which also needs the buffer
           for (; kt < kend; ++kt, ++it) {
             const int s = it % STAGES;
-            if (!__all_sync(0xffffffffu,
-                            wait_bounded(&full[s], (it / STAGES) & 1, abort_flag, lim))) {
-              ok = false;
-              break;
+            const uint32_t pf = (it / STAGES) & 1, pt = ((ch >> 1) & 1) ^ 1;
+            bool ready = mbar_try_wait(&full[s], pf);
+            if (!accumulate) ready = mbar_try_wait(&tempty[buf], pt) && ready;
+            if (!__all_sync(0xffffffffu, ready)) {
+              ready = (accumulate || wait_bounded(&tempty[buf], pt, abort_flag, lim)) &&
+                      wait_bounded(&full[s], pf, abort_flag, lim);
+              if (!__all_sync(0xffffffffu, ready)) {
+                ok = false;
+                break;
+              }
             }
             tc_fence_after();
             const uint32_t sa = base + s * S::kStageBytes;
-            const uint32_t sb = sa + P * S::kABytes;
-#pragma unroll
-            for (int ks = 0; ks < kBK / 16; ++ks) {
-#pragma unroll
-              for (int q2 = 0; q2 < Products<P>::n; ++q2) {
-                const uint64_t ad = sw64_desc(sa + Products<P>::a(q2) * S::kABytes + ks * 32);
-                const uint64_t bd = sw64_desc(sb + Products<P>::b(q2) * S::kBBytes + ks * 32);
-                tc_mma_elect(d, ad, bd, idesc, first ? 0u : 1u);
-                first = false;
-              }
+            if (tc_elect()) {
+              tc_issue_ktile<P, S::kABytes, S::kBBytes, false>(d, sa, sa + P * S::kABytes, idesc,
+                                                               accumulate);
+              tc_commit<false>(&empty[s]);
+              if (kt + 1 == kend) tc_commit<false>(&tfull[buf]);
             }
-            tc_commit_elect(&empty[s]);
+            __syncwarp();
+            accumulate = 1;
           }
-          if (ok) tc_commit_elect(&tfull[buf]);
         }
         if (!ok) break;
       }
@@ -613,8 +669,7 @@ __device__ __forceinline__ void tc_body(const Tiles& tiles, const TcRun& run) {
         for (int j = 0; j < COLS / 32; ++j) {
           float v[32];
           tmem_ld32(taddr + 32 * j, v);
-#pragma unroll
-          for (int i = 0; i < 32; ++i) sum[32 * j + i] += v[i];
+          add_drained<32>(sum + 32 * j, v);
         }
         tc_fence_before();
         __syncwarp();

@@ -58,30 +58,6 @@ HBSG_DEV void tma_load_3d_pair(uint32_t dst, const CUtensorMap* map, int c0, int
       : "memory");
 }
 
-// The pair MMA, and the commit that arrives (once) on the barrier at this
-// offset in both CTAs of the pair when all prior tensor-core work of the
-// issuing thread completes; from one elected lane of a converged warp (see
-// tc_mma_elect).
-HBSG_DEV void tc_mma_pair_elect(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p, e;\n\t.reg .b32 l;\n\t"
-      "elect.sync l|e, 0xffffffff;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "@e tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d_tmem),
-      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate));
-}
-
-HBSG_DEV void tc_commit_pair_elect(uint64_t* bar) {
-  asm volatile(
-      "{\n\t.reg .b16 m;\n\t.reg .pred e;\n\t.reg .b32 l;\n\t"
-      "elect.sync l|e, 0xffffffff;\n\t"
-      "mov.b16 m, 3;\n\t"
-      "@e tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64"
-      " [%0], m;\n\t}\n" ::"r"(smem_u32(bar))
-      : "memory");
-}
-
 template <int P, int BN, int STAGES>
 struct TcPairShape {
   static constexpr int kABytes = kBM * kBK * 2;         // 128 rows of one part
@@ -174,7 +150,7 @@ __device__ __forceinline__ void tc_pair_body(const Tiles& tiles, const TcRun& ru
   } else if (warp == 1) {
     // ---------------- MMA issuer (leader CTA only) ----------------
     // The whole warp runs the loop converged and one elected lane issues
-    // (tc_mma_elect); a wait passes only when it passed on every lane.
+    // (tc_issue_ktile); a wait passes only when it passed on every lane.
     if (leader) {
       constexpr uint32_t idesc = f16_idesc(2 * kBM, BN);
       uint32_t it = 0, ch = 0;
@@ -185,38 +161,33 @@ __device__ __forceinline__ void tc_pair_body(const Tiles& tiles, const TcRun& ru
         int kt = 0;
         for (int c = 0; c < nchunks && ok; ++c, ++ch) {
           const int buf = ch & 1;
-          if (!__all_sync(0xffffffffu,
-                          wait_bounded(&tempty[buf], ((ch >> 1) & 1) ^ 1, abort_flag, lim))) {
-            ok = false;
-            break;
-          }
-          tc_fence_after();
           const uint32_t d = tmem_base + buf * BN;
           const int kend = min(KT, kt + run.chunk_ktiles);
-          bool first = true;
+          uint32_t accumulate = 0;  // 0: the chunk's first k-tile, which also needs the buffer
           for (; kt < kend; ++kt, ++it) {
             const int s = it % STAGES;
-            if (!__all_sync(0xffffffffu,
-                            wait_bounded(&full[s], (it / STAGES) & 1, abort_flag, lim))) {
-              ok = false;
-              break;
+            const uint32_t pf = (it / STAGES) & 1, pt = ((ch >> 1) & 1) ^ 1;
+            bool ready = mbar_try_wait(&full[s], pf);
+            if (!accumulate) ready = mbar_try_wait(&tempty[buf], pt) && ready;
+            if (!__all_sync(0xffffffffu, ready)) {
+              ready = (accumulate || wait_bounded(&tempty[buf], pt, abort_flag, lim)) &&
+                      wait_bounded(&full[s], pf, abort_flag, lim);
+              if (!__all_sync(0xffffffffu, ready)) {
+                ok = false;
+                break;
+              }
             }
             tc_fence_after();
             const uint32_t sa = base + s * S::kStageBytes;
-            const uint32_t sb = sa + P * S::kABytes;
-#pragma unroll
-            for (int ks = 0; ks < kBK / 16; ++ks) {
-#pragma unroll
-              for (int q = 0; q < Products<P>::n; ++q) {
-                const uint64_t ad = sw64_desc(sa + Products<P>::a(q) * S::kABytes + ks * 32);
-                const uint64_t bd = sw64_desc(sb + Products<P>::b(q) * S::kBBytes + ks * 32);
-                tc_mma_pair_elect(d, ad, bd, idesc, first ? 0u : 1u);
-                first = false;
-              }
+            if (tc_elect()) {
+              tc_issue_ktile<P, S::kABytes, S::kBBytes, true>(d, sa, sa + P * S::kABytes, idesc,
+                                                              accumulate);
+              tc_commit<true>(&empty[s]);
+              if (kt + 1 == kend) tc_commit<true>(&tfull[buf]);
             }
-            tc_commit_pair_elect(&empty[s]);
+            __syncwarp();
+            accumulate = 1;
           }
-          if (ok) tc_commit_pair_elect(&tfull[buf]);
         }
       }
     }
@@ -249,8 +220,7 @@ __device__ __forceinline__ void tc_pair_body(const Tiles& tiles, const TcRun& ru
         for (int j = 0; j < COLS / 32; ++j) {
           float v[32];
           tmem_ld32(taddr + 32 * j, v);
-#pragma unroll
-          for (int i = 0; i < 32; ++i) sum[32 * j + i] += v[i];
+          add_drained<32>(sum + 32 * j, v);
         }
         tc_fence_before();
         __syncwarp();
