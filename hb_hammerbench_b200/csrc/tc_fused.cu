@@ -81,7 +81,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kFusedThreads, 1)
 }
 
 // A-in-TMEM form: 128 x BN tiles on single CTAs (tc_fused_ts.cuh).
-template <int P, int BN, int SA, int SB, int TSTAGES, bool SCALED>
+template <int P, int BN, int SA, int SB, int TSTAGES, int KS, bool SCALED>
 __global__ void __launch_bounds__(kTsThreads, 1)
     tc_fused_ts_kernel(const __grid_constant__ CUtensorMap tmA,
                        const __grid_constant__ CUtensorMap tmB,
@@ -90,7 +90,7 @@ __global__ void __launch_bounds__(kTsThreads, 1)
   tiles.p = &p;
   tiles.ma = &tmA;
   tiles.mb = &tmB;
-  tc_fused_ts_body<P, BN, SA, SB, TSTAGES, SCALED>(tiles, run);
+  tc_fused_ts_body<P, BN, SA, SB, TSTAGES, KS, SCALED>(tiles, run);
 }
 
 template <int P, int BN, int STAGES, int SSTAGES>
@@ -124,18 +124,18 @@ static int fused_clusters_of(bool scaled) {
   return fused_resident_clusters(k, S::kSmemBytes);
 }
 
-template <int P, int BN, int SA, int SB, int TSTAGES>
+template <int P, int BN, int SA, int SB, int TSTAGES, int KS>
 static const void* fused_ts_kernel_ptr(bool scaled) {
-  return scaled ? reinterpret_cast<const void*>(&tc_fused_ts_kernel<P, BN, SA, SB, TSTAGES, true>)
-                : reinterpret_cast<const void*>(&tc_fused_ts_kernel<P, BN, SA, SB, TSTAGES, false>);
+  return scaled ? reinterpret_cast<const void*>(&tc_fused_ts_kernel<P, BN, SA, SB, TSTAGES, KS, true>)
+                : reinterpret_cast<const void*>(&tc_fused_ts_kernel<P, BN, SA, SB, TSTAGES, KS, false>);
 }
 
-template <int P, int BN, int SA, int SB, int TSTAGES>
+template <int P, int BN, int SA, int SB, int TSTAGES, int KS>
 static cudaError_t launch_fused_ts(const CUtensorMap& a, const CUtensorMap& b,
                                    const FusedParams& p, const TcRun& run, int grid,
                                    cudaStream_t st, bool scaled) {
-  using S = TcTsShape<P, BN, SA, SB, TSTAGES>;
-  const void* k = fused_ts_kernel_ptr<P, BN, SA, SB, TSTAGES>(scaled);
+  using S = TcTsShape<P, BN, SA, SB, TSTAGES, KS>;
+  const void* k = fused_ts_kernel_ptr<P, BN, SA, SB, TSTAGES, KS>(scaled);
   static uint64_t masks[2] = {0, 0};
   if (!set_smem_once(k, S::kSmemBytes, &masks[scaled ? 1 : 0])) return cudaErrorInvalidValue;
   if (BN > 64) {  // the body's setmaxnreg split needs exactly 128 registers at launch
@@ -143,17 +143,17 @@ static cudaError_t launch_fused_ts(const CUtensorMap& a, const CUtensorMap& b,
     if (!fused_regs_ok(k, &regs_ok[scaled ? 1 : 0])) return cudaErrorInvalidConfiguration;
   }
   if (scaled)
-    tc_fused_ts_kernel<P, BN, SA, SB, TSTAGES, true><<<grid, kTsThreads, S::kSmemBytes, st>>>(a, b, p, run);
+    tc_fused_ts_kernel<P, BN, SA, SB, TSTAGES, KS, true><<<grid, kTsThreads, S::kSmemBytes, st>>>(a, b, p, run);
   else
-    tc_fused_ts_kernel<P, BN, SA, SB, TSTAGES, false><<<grid, kTsThreads, S::kSmemBytes, st>>>(a, b, p, run);
+    tc_fused_ts_kernel<P, BN, SA, SB, TSTAGES, KS, false><<<grid, kTsThreads, S::kSmemBytes, st>>>(a, b, p, run);
   return cudaGetLastError();
 }
 
 // Resident CTAs of an A-in-TMEM kernel (0 if unknown).
-template <int P, int BN, int SA, int SB, int TSTAGES>
+template <int P, int BN, int SA, int SB, int TSTAGES, int KS>
 static int fused_ts_ctas_of(bool scaled) {
-  using S = TcTsShape<P, BN, SA, SB, TSTAGES>;
-  const void* k = fused_ts_kernel_ptr<P, BN, SA, SB, TSTAGES>(scaled);
+  using S = TcTsShape<P, BN, SA, SB, TSTAGES, KS>;
+  const void* k = fused_ts_kernel_ptr<P, BN, SA, SB, TSTAGES, KS>(scaled);
   static uint64_t masks[2] = {0, 0};
   if (!set_smem_once(k, S::kSmemBytes, &masks[scaled ? 1 : 0])) return 0;
   int per_sm = 0;
@@ -179,9 +179,10 @@ struct FusedEntry {
 #define HBSG_FUSED_ENTRY(P, BN, ST, SST)                                                   \
   FusedEntry{P, BN, ST, SST, TcFusedShape<P, BN, ST, SST>::kSmemBytes, 0, 2 * kBM,        \
              kFusedThreads, &launch_fused<P, BN, ST, SST>, &fused_clusters_of<P, BN, ST, SST>},
-#define HBSG_FUSED_TS_ENTRY(P, BN, SA, SB, TST)                                               \
-  FusedEntry{P, BN, SA, SB, TcTsShape<P, BN, SA, SB, TST>::kSmemBytes, 1, kBM, kTsThreads,     \
-             &launch_fused_ts<P, BN, SA, SB, TST>, &fused_ts_ctas_of<P, BN, SA, SB, TST>},
+#define HBSG_FUSED_TS_ENTRY(P, BN, SA, SB, TST, KS)                                           \
+  FusedEntry{P, BN, SA, SB, TcTsShape<P, BN, SA, SB, TST, KS>::kSmemBytes, 1, kBM, kTsThreads, \
+             &launch_fused_ts<P, BN, SA, SB, TST, KS>,                                         \
+             &fused_ts_ctas_of<P, BN, SA, SB, TST, KS>},
 // CTA-pair tiles first (the grouped plans' fused table, grouped.cu, holds
 // these only), then the A-in-TMEM tiles
 static const FusedEntry kFused[] = {HBSG_FUSED_TILE_LIST(HBSG_FUSED_ENTRY)

@@ -44,8 +44,8 @@
 //   warp 2       lane 0: TMA loads of the B parts
 //   warp 3       no role
 //   warps 4-11   A converters: thread = row 32 (warp % 4) + lane; warps 4-7
-//                convert the even k-tiles, warps 8-11 the odd ones, so one
-//                group's loads overlap the other's stores
+//                convert the even steps (of one or two k-tiles), warps 8-11
+//                the odd ones, so one group's loads overlap the other's stores
 //   warps 12-15  epilogue (TMEM lane quadrant warp % 4, all BN columns)
 // Every wait is bounded as in the other tensor-core bodies. The TMA loads use
 // no cluster multicast.
@@ -55,15 +55,15 @@
 
 namespace hbsg {
 
-// (parts, BN, A staging stages, B parts stages, TMEM A slots)
+// (parts, BN, A staging stages, B parts stages, TMEM A slots, k-tiles per step)
 #define HBSG_FUSED_TS_TILE_LIST(X) \
-  X(3, 64, 6, 8, 8)                \
-  X(2, 64, 8, 8, 12)               \
-  X(3, 128, 4, 5, 4)               \
-  X(2, 128, 6, 6, 8)
+  X(3, 64, 4, 4, 4, 2)             \
+  X(2, 64, 4, 6, 6, 2)             \
+  X(3, 128, 4, 5, 4, 1)            \
+  X(2, 128, 6, 6, 8, 1)
 
 static constexpr int kTsThreads = 512;
-static constexpr int kTsAGroups = 2;  // A converter groups of 4 warps, alternating k-tiles
+static constexpr int kTsAGroups = 2;  // A converter groups of 4 warps, alternating steps
 // Tiles wider than 64 columns: the epilogue warpgroup holds BN FP32 sums per
 // thread, so setmaxnreg moves registers to it from the other three
 // warpgroups (3 x 128 x 112 + 128 x 176 = 65536, the block's launch
@@ -72,25 +72,35 @@ static constexpr int kTsRegsLow = 112;
 static constexpr int kTsRegsHigh = 176;
 static_assert(3 * 128 * kTsRegsLow + 128 * kTsRegsHigh == 65536, "register split");
 
-template <int P, int BN, int SA, int SB, int TSTAGES>
+// KS: k-tiles per pipeline step. Stages, TMEM slots and barrier phases hold one
+// step, so two k-tiles halve the waits, commits and arrivals per MMA where
+// both fit (BN = 64).
+template <int P, int BN, int SA, int SB, int TSTAGES, int KS>
 struct TcTsShape {
-  static constexpr int kSABytes = kBM * kBK * 4;  // one FP32 A staging stage
+  static constexpr int kSABytes = kBM * kBK * 4;  // FP32 A of one k-tile
   static constexpr int kBPart = BN * kBK * 2;     // one B part of one k-tile
-  static constexpr int kSBBytes = P * kBPart;     // one B parts stage
-  static constexpr int kBRingOff = SA * kSABytes;
-  static constexpr int kACols = P * (kBK / 2);  // TMEM columns of one slot
+  static constexpr int kSBBytes = P * kBPart;     // B parts of one k-tile
+  static constexpr int kSAStage = KS * kSABytes;  // one FP32 A staging stage
+  static constexpr int kSBStage = KS * kSBBytes;  // one B parts stage
+  static constexpr int kBRingOff = SA * kSAStage;
+  static constexpr int kATile = P * (kBK / 2);  // TMEM columns of one k-tile's A parts
+  static constexpr int kACols = KS * kATile;    // of one slot
+  // B stage and TMEM slot of a step are the same index: the MMAs release both
+  // with one commit on one barrier
+  static constexpr bool kOneEmpty = SB == TSTAGES;
   static constexpr int kAColBase = 2 * BN;
   static constexpr int kTmemCols = kAColBase + TSTAGES * kACols;
   static constexpr int kAllocCols = kTmemCols <= 32 ? 32 : kTmemCols <= 64 ? 64 : kTmemCols <= 128 ? 128 : kTmemCols <= 256 ? 256 : 512;
   static constexpr int kBarBytes = 8 * (2 * SA + 2 * SB + 2 * TSTAGES + 4) + 16;
   static constexpr int kColExpBytes = 4 * 4 * BN;  // 4 epilogue warps x BN column exponents
-  static constexpr int kBarOff = kBRingOff + SB * kSBBytes;
+  static constexpr int kBarOff = kBRingOff + SB * kSBStage;
   static constexpr int kSmemBytes = 1024 + kBarOff + kBarBytes + kColExpBytes;
   static_assert(kSmemBytes <= 232448, "shared memory");
   static_assert(kTmemCols <= 512, "tensor memory");
   static_assert(BN % 32 == 0 && BN >= 32 && BN <= 256, "UMMA N (M = 128) and 32-column stores");
   static_assert(TSTAGES % kTsAGroups == 0 && SA % kTsAGroups == 0,
-                "each converter group owns whole TMEM slots and staging stages");
+                "each converter group owns whole TMEM slots and staging stages: a group waits on "
+                "one barrier phase in two otherwise, and a parity wait cannot tell them apart");
   static_assert(kSABytes % 1024 == 0 && kBRingOff % 1024 == 0 && kBPart % 512 == 0,
                 "staging keeps the 128-byte swizzle's 1024-byte and the parts' 512-byte alignment");
 };
@@ -117,9 +127,9 @@ HBSG_DEV void tc_mma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32
       "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate));
 }
 
-template <int P, int BN, int SA, int SB, int TSTAGES, bool SCALED, class Tiles>
+template <int P, int BN, int SA, int SB, int TSTAGES, int KS, bool SCALED, class Tiles>
 __device__ __forceinline__ void tc_fused_ts_body(const Tiles& tiles, const TcRun& run) {
-  using S = TcTsShape<P, BN, SA, SB, TSTAGES>;
+  using S = TcTsShape<P, BN, SA, SB, TSTAGES, KS>;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
@@ -191,24 +201,34 @@ __device__ __forceinline__ void tc_fused_ts_body(const Tiles& tiles, const TcRun
         const CUtensorMap* map = a_role ? w.ma : w.mb;
         if (t == (int)blockIdx.x)
           asm volatile("prefetch.tensormap [%0];\n" ::"l"(reinterpret_cast<uint64_t>(map)) : "memory");
-        for (int kt = 0; kt < w.KT; ++kt, ++it) {
+        for (int kt = 0; kt < w.KT; kt += KS, ++it) {
           const int k0 = (w.kt0 + kt) * kBK;
+          const int nk = min(KS, w.KT - kt);  // k-tiles of this step
           if (a_role) {
             const int s = it % SA;
             if (!wait_bounded_hint(&sempty[s], ((it / SA) & 1) ^ 1, abort_flag, lim)) {
               ok = false;
               break;
             }
-            mbar_arrive_expect_tx(&sfull[s], S::kSABytes);
-            tma_load_2d(base + s * S::kSABytes, map, k0, w.m0, &sfull[s]);
+            mbar_arrive_expect_tx(&sfull[s], nk * S::kSABytes);
+#pragma unroll
+            for (int e = 0; e < KS; ++e)
+              if (e < nk)
+                tma_load_2d(base + s * S::kSAStage + e * S::kSABytes, map, k0 + e * kBK, w.m0,
+                            &sfull[s]);
           } else {
             const int s = it % SB;
-            if (!wait_bounded_hint(&bempty[s], ((it / SB) & 1) ^ 1, abort_flag, lim)) {
+            if (!wait_bounded_hint(S::kOneEmpty ? &aempty[s] : &bempty[s], ((it / SB) & 1) ^ 1,
+                                   abort_flag, lim)) {
               ok = false;
               break;
             }
-            mbar_arrive_expect_tx(&bfull[s], S::kSBBytes);
-            tma_load_3d(base + S::kBRingOff + s * S::kSBBytes, map, k0, w.n0, 0, &bfull[s]);
+            mbar_arrive_expect_tx(&bfull[s], nk * S::kSBBytes);
+#pragma unroll
+            for (int e = 0; e < KS; ++e)
+              if (e < nk)
+                tma_load_3d(base + S::kBRingOff + s * S::kSBStage + e * S::kSBBytes, map,
+                            k0 + e * kBK, w.n0, 0, &bfull[s]);
           }
         }
       }
@@ -220,61 +240,78 @@ __device__ __forceinline__ void tc_fused_ts_body(const Tiles& tiles, const TcRun
     // counts as passed only when it passed on all lanes. Measured per k-tile of
     // 65536 x 64 x 4096 (6 products, cycles by role counters): 381 of MMA issue
     // (its tensor-core time) but 684 of waits, commits and loop around it, and
-    // the converters waiting for this warp; 848 in all in this form.
+    // the converters waiting for this warp; 848 in all in this form, and with
+    // two k-tiles per step 345 -> 323 -> 290 us for the call.
     constexpr uint32_t idesc = f16_idesc(kBM, BN);
     uint32_t it = 0, ch = 0;
     bool ok = true;
     for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x) {
-      const TileWork w = tiles.get(t);
-      const int KT = w.KT;
-      const int nchunks = (KT + run.chunk_ktiles - 1) / run.chunk_ktiles;
-      int kt = 0;
-      for (int c = 0; c < nchunks && ok; ++c, ++ch) {
-        const int buf = ch & 1;
-        const uint32_t d = tmem_base + buf * BN;
-        const int kend = min(KT, kt + run.chunk_ktiles);
-        uint32_t accumulate = 0;  // 0: the chunk's first k-tile, which also needs the buffer
-        for (; kt < kend; ++kt, ++it) {
-          const int sb = it % SB;
-          const int j = it % TSTAGES;
-          const uint32_t pb = (it / SB) & 1, pa = (it / TSTAGES) & 1, pt = ((ch >> 1) & 1) ^ 1;
-          const bool rb = mbar_try_wait(&bfull[sb], pb);
-          bool ready = mbar_try_wait(&afull[j], pa) && rb;
-          if (!accumulate) ready = mbar_try_wait(&tempty[buf], pt) && ready;
+      const int KT = tiles.get(t).KT;
+      int left = 0;  // k-tiles left in the chunk
+      uint32_t d = 0, accumulate = 0;
+      for (int kt = 0; kt < KT && ok; kt += KS, ++it) {
+        const int sb = it % SB;
+        const int j = it % TSTAGES;
+        const uint32_t pb = (it / SB) & 1, pa = (it / TSTAGES) & 1;
+        // a chunk that starts with this step needs its accumulator buffer too
+        const uint32_t pt = ((ch >> 1) & 1) ^ 1;
+        const bool rb = mbar_try_wait(&bfull[sb], pb);
+        bool ready = mbar_try_wait(&afull[j], pa) && rb;
+        if (left == 0) ready = mbar_try_wait(&tempty[ch & 1], pt) && ready;
+        if (!__all_sync(0xffffffffu, ready)) {
+          ready = (left != 0 || wait_bounded(&tempty[ch & 1], pt, abort_flag, lim)) &&
+                  wait_bounded(&bfull[sb], pb, abort_flag, lim) &&
+                  wait_bounded(&afull[j], pa, abort_flag, lim);
           if (!__all_sync(0xffffffffu, ready)) {
-            ready = (accumulate || wait_bounded(&tempty[buf], pt, abort_flag, lim)) &&
-                    wait_bounded(&bfull[sb], pb, abort_flag, lim) &&
-                    wait_bounded(&afull[j], pa, abort_flag, lim);
-            if (!__all_sync(0xffffffffu, ready)) {
-              ok = false;
-              break;
-            }
+            ok = false;
+            break;
           }
-          tc_fence_after();
-          const uint32_t ta = tmem_base + S::kAColBase + j * S::kACols;
+        }
+        tc_fence_after();
+        const uint32_t ta0 = tmem_base + S::kAColBase + j * S::kACols;
+        const uint64_t bd0 = sw64_desc(base + S::kBRingOff + sb * S::kSBStage);
+#pragma unroll
+        for (int e = 0; e < KS; ++e) {
+          if (kt + e >= KT) break;
+          if (left == 0) {
+            if (e > 0) {  // (a chunk starting inside the step: its buffer was not probed above)
+              const bool got = wait_bounded(&tempty[ch & 1], ((ch >> 1) & 1) ^ 1, abort_flag, lim);
+              if (!__all_sync(0xffffffffu, got)) {
+                ok = false;
+                break;
+              }
+              tc_fence_after();
+            }
+            d = tmem_base + (ch & 1) * BN;
+            accumulate = 0;
+            left = min(run.chunk_ktiles, KT - kt - e);
+          }
+          --left;
           if (tc_elect()) {
-            const uint64_t bd = sw64_desc(base + S::kBRingOff + sb * S::kSBBytes);
 #pragma unroll
             for (int ks = 0; ks < kBK / 16; ++ks) {
 #pragma unroll
               for (int q = 0; q < Products<P>::n; ++q)
-                tc_mma_ts(d, ta + Products<P>::a(q) * (kBK / 2) + ks * 8,
-                          bd + ((Products<P>::b(q) * S::kBPart + ks * 32) >> 4), idesc,
-                          ks == 0 && q == 0 ? accumulate : 1u);
+                tc_mma_ts(d, ta0 + e * S::kATile + Products<P>::a(q) * (kBK / 2) + ks * 8,
+                          bd0 + ((e * S::kSBBytes + Products<P>::b(q) * S::kBPart + ks * 32) >> 4),
+                          idesc, ks == 0 && q == 0 ? accumulate : 1u);
             }
-            tc_commit<false>(&bempty[sb]);
-            tc_commit<false>(&aempty[j]);
-            if (kt + 1 == kend) tc_commit<false>(&tfull[buf]);
+            if (e == KS - 1 || kt + e + 1 == KT) {  // the step's last k-tile
+              tc_commit<false>(&aempty[j]);
+              if constexpr (!S::kOneEmpty) tc_commit<false>(&bempty[sb]);
+            }
+            if (left == 0) tc_commit<false>(&tfull[ch & 1]);
           }
           __syncwarp();
           accumulate = 1;
+          if (left == 0) ++ch;
         }
       }
     }
   } else if (warp >= 4 && warp < 4 + 4 * kTsAGroups) {
     // ---------------- A converters ----------------
     // thread = tile row 32 q + lane (its TMEM lane); group g converts the
-    // k-tiles it with it % 2 == g: eight 16-byte staging loads (then the
+    // steps it with it % 2 == g, per k-tile: eight 16-byte staging loads (then the
     // staging stage is released), the split of 32 values, P x 16 TMEM columns
     const int q = warp & 3;
     const int g = (warp - 4) >> 2;
@@ -289,49 +326,59 @@ __device__ __forceinline__ void tc_fused_ts_body(const Tiles& tiles, const TcRun
         const int m = w.m0 + r;
         ex = m < w.M ? exp_from_maxbits(w.rowmax[m]) : 0;
       }
-      for (int kt = 0; kt < w.KT; ++kt, ++it) {
+      for (int kt = 0; kt < w.KT; kt += KS, ++it) {
         if ((int)(it % kTsAGroups) != g) continue;
         const int s = it % SA;
         const int j = it % TSTAGES;
+        const int nk = min(KS, w.KT - kt);
         if (!wait_bounded_hint(&sfull[s], (it / SA) & 1, abort_flag, lim)) {
           ok = false;
           break;
         }
-        const uint8_t* fa = smem + s * S::kSABytes;
-        float v[4][8];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const float4 a0 = *reinterpret_cast<const float4*>(fa + sw128_offset(r, 2 * u));
-          const float4 a1 = *reinterpret_cast<const float4*>(fa + sw128_offset(r, 2 * u + 1));
-          v[u][0] = a0.x; v[u][1] = a0.y; v[u][2] = a0.z; v[u][3] = a0.w;
-          v[u][4] = a1.x; v[u][5] = a1.y; v[u][6] = a1.z; v[u][7] = a1.w;
-        }
-        uint4 o[4][P];
+        for (int e = 0; e < KS; ++e) {
+          if (e >= nk) break;
+          const uint8_t* fa = smem + s * S::kSAStage + e * S::kSABytes;
+          float v[4][8];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) split8<P, SCALED>(v[u], ex, o[u]);
-        // the staging values are in registers (the split used them): the
-        // stage may be reloaded by the TMA
-        fence_proxy_async_smem();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&sempty[s]);
-        // the slot is free once the MMAs that read it (k-tile it - TSTAGES)
-        // completed
-        if (!wait_bounded_hint(&aempty[j], ((it / TSTAGES) & 1) ^ 1, abort_flag, lim)) {
-          ok = false;
-          break;
-        }
-        tc_fence_after();
-        const uint32_t ta = trow + j * S::kACols;
+          for (int u = 0; u < 4; ++u) {
+            const float4 a0 = *reinterpret_cast<const float4*>(fa + sw128_offset(r, 2 * u));
+            const float4 a1 = *reinterpret_cast<const float4*>(fa + sw128_offset(r, 2 * u + 1));
+            v[u][0] = a0.x; v[u][1] = a0.y; v[u][2] = a0.z; v[u][3] = a0.w;
+            v[u][4] = a1.x; v[u][5] = a1.y; v[u][6] = a1.z; v[u][7] = a1.w;
+          }
+          uint4 o[4][P];
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
+          for (int u = 0; u < 4; ++u) split8<P, SCALED>(v[u], ex, o[u]);
+          if (e + 1 == nk) {
+            // the staging values are in registers (the split used them): the
+            // stage may be reloaded by the TMA
+            fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&sempty[s]);
+          }
+          if (e == 0) {
+            // the slot is free once the MMAs that read it (step it - TSTAGES)
+            // completed
+            if (!wait_bounded_hint(&aempty[j], ((it / TSTAGES) & 1) ^ 1, abort_flag, lim)) {
+              ok = false;
+              break;
+            }
+            tc_fence_after();
+          }
+          const uint32_t ta = trow + j * S::kACols + e * S::kATile;
 #pragma unroll
-          for (int p = 0; p < P; ++p) {
-            const uint32_t reg[8] = {o[2 * h][p].x,     o[2 * h][p].y,     o[2 * h][p].z,
-                                     o[2 * h][p].w,     o[2 * h + 1][p].x, o[2 * h + 1][p].y,
-                                     o[2 * h + 1][p].z, o[2 * h + 1][p].w};
-            tmem_st8(ta + p * (kBK / 2) + h * (kBK / 4), reg);
+          for (int h = 0; h < 2; ++h) {
+#pragma unroll
+            for (int p = 0; p < P; ++p) {
+              const uint32_t reg[8] = {o[2 * h][p].x,     o[2 * h][p].y,     o[2 * h][p].z,
+                                       o[2 * h][p].w,     o[2 * h + 1][p].x, o[2 * h + 1][p].y,
+                                       o[2 * h + 1][p].z, o[2 * h + 1][p].w};
+              tmem_st8(ta + p * (kBK / 2) + h * (kBK / 4), reg);
+            }
           }
         }
+        if (!ok) break;
         tmem_wait_st();
         tc_fence_before();
         __syncwarp();
