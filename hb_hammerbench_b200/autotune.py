@@ -65,9 +65,9 @@ def cache_path() -> str:
 
 
 def shape_key(m: int, n: int, k: int, variant: str) -> str:
-    def b(x):
-        return max(0, math.ceil(math.log2(max(1, x))))
-    return f"{variant}:m{b(m)}:n{b(n)}:k{b(k)}"
+    # ceil(log2(x)) of each dimension, 0 for x < 1
+    return (f"{variant}:m{(max(1, m) - 1).bit_length()}:n{(max(1, n) - 1).bit_length()}"
+            f":k{(max(1, k) - 1).bit_length()}")
 
 
 def grouped_key(dims, variant: str) -> str:

@@ -21,7 +21,7 @@ import numpy as np
 import torch
 
 from ._lib import check, lib
-from .sgemm import _check_f32_cuda, _ptr, _stream
+from .sgemm import _check_f32_cuda, _on_device
 
 FIELDS = ("s", "strike", "r", "v", "t", "call", "put", "unused")
 RECORD_FLOATS = 8
@@ -50,9 +50,8 @@ def price(records: torch.Tensor) -> torch.Tensor:
     _check_f32_cuda("records", records)
     if records.dim() != 2 or records.shape[1] != RECORD_FLOATS or not records.is_contiguous():
         raise ValueError("records must be a contiguous (n, 8) float32 tensor")
-    with torch.cuda.device(records.device):
-        check(lib().hbsg_blackscholes(_ptr(records), records.shape[0], _stream()),
-              "hbsg_blackscholes")
+    check(_on_device(records.device, lib().hbsg_blackscholes, records.data_ptr(),
+                     records.shape[0]), "hbsg_blackscholes")
     return records
 
 
@@ -73,8 +72,7 @@ def price_arrays(s: torch.Tensor, strike: torch.Tensor, r: torch.Tensor, v: torc
         _check_f32_cuda(name, x)
         if not x.is_contiguous() or x.numel() != n:
             raise ValueError(f"{name} must be a contiguous array of {n} floats")
-    with torch.cuda.device(s.device):
-        check(lib().hbsg_blackscholes_arrays(*[_ptr(x) for x in ins], _ptr(call), _ptr(put), n,
-                                             _stream()),
-              "hbsg_blackscholes_arrays")
+    check(_on_device(s.device, lib().hbsg_blackscholes_arrays, s.data_ptr(), strike.data_ptr(),
+                     r.data_ptr(), v.data_ptr(), t.data_ptr(), call.data_ptr(), put.data_ptr(), n),
+          "hbsg_blackscholes_arrays")
     return call, put

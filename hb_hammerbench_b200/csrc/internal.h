@@ -133,6 +133,24 @@ static constexpr int kMaxDevices = 64;
 // no sm_100 device is current (or its ordinal is >= kMaxDevices).
 int current_device_sms(int* device_out);
 
+// A per-device figure of a kernel that the runtime takes microseconds to work
+// out (resident CTAs or clusters, for its fixed block and shared memory),
+// asked for once per device: `query` runs until it gives a positive value.
+struct DeviceCache {
+  int value[kMaxDevices];
+};
+template <class Query>
+int cached_per_device(DeviceCache* cache, Query query) {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return query();
+  int v = __atomic_load_n(&cache->value[dev], __ATOMIC_RELAXED);
+  if (v <= 0) {
+    v = query();
+    if (v > 0) __atomic_store_n(&cache->value[dev], v, __ATOMIC_RELAXED);
+  }
+  return v;
+}
+
 // Sets a kernel's dynamic shared memory limit once per device (one bit of
 // *device_mask per device ordinal).
 bool set_smem_once(const void* func, int bytes, uint64_t* device_mask);

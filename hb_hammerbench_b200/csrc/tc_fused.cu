@@ -120,8 +120,10 @@ static int fused_clusters_of(bool scaled) {
   using S = TcFusedShape<P, BN, STAGES, SSTAGES>;
   const void* k = fused_kernel_ptr<P, BN, STAGES, SSTAGES>(scaled);
   static uint64_t masks[2] = {0, 0};
+  static DeviceCache resident[2];
   if (!set_smem_once(k, S::kSmemBytes, &masks[scaled ? 1 : 0])) return 0;
-  return fused_resident_clusters(k, S::kSmemBytes);
+  return cached_per_device(&resident[scaled ? 1 : 0],
+                           [&] { return fused_resident_clusters(k, S::kSmemBytes); });
 }
 
 template <int P, int BN, int SA, int SB, int TSTAGES, int KS>
@@ -156,12 +158,16 @@ static int fused_ts_ctas_of(bool scaled) {
   const void* k = fused_ts_kernel_ptr<P, BN, SA, SB, TSTAGES, KS>(scaled);
   static uint64_t masks[2] = {0, 0};
   if (!set_smem_once(k, S::kSmemBytes, &masks[scaled ? 1 : 0])) return 0;
-  int per_sm = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kTsThreads, S::kSmemBytes) !=
-      cudaSuccess) {
-    cudaGetLastError();
-    return 0;
-  }
+  static DeviceCache resident[2];
+  const int per_sm = cached_per_device(&resident[scaled ? 1 : 0], [&] {
+    int n = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, kTsThreads, S::kSmemBytes) !=
+        cudaSuccess) {
+      cudaGetLastError();
+      return 0;
+    }
+    return n;
+  });
   int sms = current_device_sms(nullptr);
   return sms > 0 ? per_sm * sms : 0;
 }

@@ -246,23 +246,26 @@ static int pair_clusters(bool scaled) {
   using S = TcPairShape<P, BN, STAGES>;
   const void* k = scaled ? reinterpret_cast<const void*>(&tc_pair_kernel<P, BN, STAGES, true>)
                          : reinterpret_cast<const void*>(&tc_pair_kernel<P, BN, STAGES, false>);
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(2, 1, 1);
-  cfg.blockDim = dim3(320, 1, 1);
-  cfg.dynamicSmemBytes = S::kSmemBytes;
-  cudaLaunchAttribute attr;
-  attr.id = cudaLaunchAttributeClusterDimension;
-  attr.val.clusterDim.x = 2;
-  attr.val.clusterDim.y = 1;
-  attr.val.clusterDim.z = 1;
-  cfg.attrs = &attr;
-  cfg.numAttrs = 1;
-  int n = 0;
-  if (cudaOccupancyMaxActiveClusters(&n, k, &cfg) != cudaSuccess) {
-    cudaGetLastError();
-    return 0;
-  }
-  return n;
+  static DeviceCache resident[2];
+  return cached_per_device(&resident[scaled ? 1 : 0], [&] {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(2, 1, 1);
+    cfg.blockDim = dim3(320, 1, 1);
+    cfg.dynamicSmemBytes = S::kSmemBytes;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = 2;
+    attr.val.clusterDim.y = 1;
+    attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, k, &cfg) != cudaSuccess) {
+      cudaGetLastError();
+      return 0;
+    }
+    return n;
+  });
 }
 
 bool tc_make_parts_map(void* map, const void* parts, int P, int rows, int Kp, int box_rows) {

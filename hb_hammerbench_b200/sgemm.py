@@ -18,12 +18,27 @@ import ctypes
 
 import torch
 
-from . import _lib
+from . import _lib, autotune
 from ._lib import Config, HbsgError, TileInfo, check, lib  # noqa: F401
 
+# The entry points below are called in loops of small products, where this
+# file's own time per call is what counts (a 1024^3 6-product call: 37 us of
+# host time against 27 us on the GPU). They hand plain integers to ctypes, ask
+# torch for the raw stream, switch devices only when the tensors are on
+# another one, and keep the ctypes form of a schedule by its values.
 
-def _stream() -> ctypes.c_void_p:
-    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+
+def _stream() -> int:
+    return torch.cuda.current_stream().cuda_stream
+
+
+def _on_device(device: torch.device, fn, *args) -> int:
+    """fn(*args, stream) on `device` and its current stream."""
+    index = device.index
+    if torch._C._cuda_getDevice() == index:
+        return fn(*args, torch._C._cuda_getCurrentRawStream(index))
+    with torch.cuda.device(index):
+        return fn(*args, torch._C._cuda_getCurrentRawStream(index))
 
 
 def _variant(v) -> int:
@@ -32,8 +47,8 @@ def _variant(v) -> int:
     return int(v)
 
 
-def _ptr(t: torch.Tensor | None) -> ctypes.c_void_p:
-    return ctypes.c_void_p(0 if t is None else t.data_ptr())
+def _ptr(t: torch.Tensor | None) -> int | None:
+    return None if t is None else t.data_ptr()
 
 
 def _check_f32_cuda(name: str, t: torch.Tensor) -> None:
@@ -41,12 +56,22 @@ def _check_f32_cuda(name: str, t: torch.Tensor) -> None:
         raise TypeError(f"{name} must be a float32 CUDA tensor")
 
 
+_configs: dict = {}  # a schedule's items -> its ctypes pointer (the library only reads it)
+
+
 def _config(cfg) -> ctypes.POINTER(Config) | None:
     if cfg is None:
         return None
-    if isinstance(cfg, dict):
-        cfg = Config(**cfg)
-    return ctypes.pointer(cfg)
+    if not isinstance(cfg, dict):
+        return ctypes.pointer(cfg)
+    key = tuple(cfg.items())
+    p = _configs.get(key)
+    if p is None:
+        p = ctypes.pointer(Config(**cfg))
+        if len(_configs) >= 256:
+            _configs.clear()
+        _configs[key] = p
+    return p
 
 
 def sgemm_workspace_size(n: int, niter: int, variant="ffma") -> int:
@@ -83,17 +108,21 @@ def sgemm(mat1: torch.Tensor, mat2: torch.Tensor, result: torch.Tensor | None = 
         result = torch.empty_like(mat1)
     _check_f32_cuda("result", result)
     v = _variant(variant)
-    with torch.cuda.device(mat1.device):
-        if v == _lib.FFMA and workspace is None:
-            st = lib().hbsg_sgemm(_ptr(mat1), _ptr(mat2), _ptr(result), n, niter, _stream())
-            check(st, "hbsg_sgemm")
-        else:
-            need = sgemm_workspace_size(n, niter, v)
-            ws = _workspace(need, mat1.device, workspace)
-            st = lib().hbsg_sgemm_variant(_ptr(mat1), _ptr(mat2), _ptr(result), n, niter, v,
-                                          _ptr(ws), need, _stream())
-            check(st, "hbsg_sgemm_variant")
+    if v == _lib.FFMA and workspace is None:
+        check(_on_device(mat1.device, lib().hbsg_sgemm, mat1.data_ptr(), mat2.data_ptr(),
+                         result.data_ptr(), n, niter), "hbsg_sgemm")
+        return result
+
+    def call(stream):
+        need = sgemm_workspace_size(n, niter, v)
+        ws = _workspace(need, mat1.device, workspace)
+        return lib().hbsg_sgemm_variant(_ptr(mat1), _ptr(mat2), _ptr(result), n, niter, v,
+                                        _ptr(ws), need, stream)
+    check(_on_device(mat1.device, call), "hbsg_sgemm_variant")
     return result
+
+
+_VARIANT_NAMES = {v: name for name, v in _lib.VARIANTS.items()}
 
 
 def resolve_config(m: int, n: int, k: int, variant, trans: bool, config):
@@ -102,10 +131,9 @@ def resolve_config(m: int, n: int, k: int, variant, trans: bool, config):
     tuner measures those), else None (the library heuristic)."""
     if config is not None or trans:
         return config
-    from . import autotune
     if not autotune.enabled():
         return None
-    name = variant if isinstance(variant, str) else {v: k_ for k_, v in _lib.VARIANTS.items()}[int(variant)]
+    name = variant if isinstance(variant, str) else _VARIANT_NAMES[int(variant)]
     return autotune.lookup(m, n, k, name.lower())
 
 
@@ -120,8 +148,12 @@ def gemm(a: torch.Tensor, b: torch.Tensor, c: torch.Tensor | None = None, varian
     _check_f32_cuda("b", b)
     if a.dim() != 2 or b.dim() != 2 or a.stride(1) != 1 or b.stride(1) != 1:
         raise ValueError("a and b must be 2-D with unit inner stride")
-    m, k = (a.shape[1], a.shape[0]) if trans_a else (a.shape[0], a.shape[1])
-    kb, n = (b.shape[1], b.shape[0]) if trans_b else (b.shape[0], b.shape[1])
+    m, k = a.shape
+    kb, n = b.shape
+    if trans_a:
+        m, k = k, m
+    if trans_b:
+        kb, n = n, kb
     if k != kb:
         raise ValueError(f"inner dimensions differ: {k} vs {kb}")
     if c is None:
@@ -131,15 +163,16 @@ def gemm(a: torch.Tensor, b: torch.Tensor, c: torch.Tensor | None = None, varian
         raise ValueError("c must be m x n with unit inner stride")
     v = _variant(variant)
     cfgp = _config(resolve_config(m, n, k, variant, trans_a or trans_b, config))
-    with torch.cuda.device(a.device):
-        need = int(lib().hbsg_gemm_workspace_size_for(int(trans_a), int(trans_b), m, n, k,
-                                                      _ptr(a), a.stride(0), _ptr(b), b.stride(0),
-                                                      v, cfgp))
+    ta, tb = int(trans_a), int(trans_b)
+    pa, lda, pb, ldb = a.data_ptr(), a.stride(0), b.data_ptr(), b.stride(0)
+    l = lib()
+
+    def call(stream):
+        need = l.hbsg_gemm_workspace_size_for(ta, tb, m, n, k, pa, lda, pb, ldb, v, cfgp)
         ws = _workspace(need, a.device, workspace)
-        st = lib().hbsg_gemm_ex(int(trans_a), int(trans_b), m, n, k, _ptr(a), a.stride(0),
-                                _ptr(b), b.stride(0), _ptr(c), c.stride(0), v, cfgp,
-                                _ptr(ws), need, _stream())
-        check(st, "hbsg_gemm_ex")
+        return l.hbsg_gemm_ex(ta, tb, m, n, k, pa, lda, pb, ldb, c.data_ptr(), c.stride(0), v,
+                              cfgp, _ptr(ws), need, stream)
+    check(_on_device(a.device, call), "hbsg_gemm_ex")
     return c
 
 
@@ -171,12 +204,9 @@ class GroupedPlan:
         self.As, self.Bs, self.Cs = list(As), list(Bs), list(Cs)
         self.variant = _variant(variant)
         self._arr = _problems(self.As, self.Bs, self.Cs)
-        if config is None and self.As:
-            from . import autotune
-            if autotune.enabled():
-                name = {v: k_ for k_, v in _lib.VARIANTS.items()}[self.variant]
-                dims = [(a.shape[0], b.shape[1], a.shape[1]) for a, b in zip(self.As, self.Bs)]
-                config = autotune.lookup_grouped(dims, name)
+        if config is None and self.As and autotune.enabled():
+            dims = [(a.shape[0], b.shape[1], a.shape[1]) for a, b in zip(self.As, self.Bs)]
+            config = autotune.lookup_grouped(dims, _VARIANT_NAMES[self.variant])
         self.config = config
         self._cfg = _config(config)
         dev = self.As[0].device if self.As else torch.device("cuda")
@@ -193,8 +223,10 @@ class GroupedPlan:
         self.device = dev
 
     def run(self):
-        with torch.cuda.device(self.device):
-            check(lib().hbsg_grouped_run(self._plan, _stream()), "hbsg_grouped_run")
+        device = self.device
+        if device.index is None:  # a plan of no problems
+            device = torch.device("cuda", torch.cuda.current_device())
+        check(_on_device(device, lib().hbsg_grouped_run, self._plan), "hbsg_grouped_run")
         return self.Cs
 
     def close(self):
@@ -289,7 +321,6 @@ def jacobi(a0: torch.Tensor, nx: int, ny: int, nz: int, c0: int = 2, c1: int = 4
     _check_f32_cuda("out", out)
     if not out.is_contiguous() or out.numel() != a0.numel():
         raise ValueError("out must be a contiguous grid of nx*ny*nz floats")
-    with torch.cuda.device(a0.device):
-        check(lib().hbsg_jacobi(c0, c1, _ptr(a0), _ptr(out), nx, ny, nz, _stream()),
-              "hbsg_jacobi")
+    check(_on_device(a0.device, lib().hbsg_jacobi, c0, c1, a0.data_ptr(), out.data_ptr(), nx, ny,
+                     nz), "hbsg_jacobi")
     return out
