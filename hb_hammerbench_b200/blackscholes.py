@@ -55,23 +55,25 @@ def price(records: torch.Tensor) -> torch.Tensor:
     return records
 
 
+def _check_arrays(n: int, named) -> None:
+    f32 = torch.float32
+    for name, x in named:
+        if x.dtype != f32 or not x.is_cuda:
+            _check_f32_cuda(name, x)
+        if x.numel() != n or not x.is_contiguous():
+            raise ValueError(f"{name} must be a contiguous array of {n} floats")
+
+
 def price_arrays(s: torch.Tensor, strike: torch.Tensor, r: torch.Tensor, v: torch.Tensor,
                  t: torch.Tensor, call: torch.Tensor | None = None,
                  put: torch.Tensor | None = None):
     """Price options held as separate float32 CUDA arrays
     (hbsg_blackscholes_arrays); returns (call, put)."""
-    ins = (s, strike, r, v, t)
     n = s.numel()
-    for name, x in zip(FIELDS, ins):
-        _check_f32_cuda(name, x)
-        if not x.is_contiguous() or x.numel() != n:
-            raise ValueError(f"{name} must be a contiguous array of {n} floats")
+    _check_arrays(n, zip(FIELDS, (s, strike, r, v, t)))
     call = torch.empty_like(s) if call is None else call
     put = torch.empty_like(s) if put is None else put
-    for name, x in (("call", call), ("put", put)):
-        _check_f32_cuda(name, x)
-        if not x.is_contiguous() or x.numel() != n:
-            raise ValueError(f"{name} must be a contiguous array of {n} floats")
+    _check_arrays(n, (("call", call), ("put", put)))
     check(_on_device(s.device, lib().hbsg_blackscholes_arrays, s.data_ptr(), strike.data_ptr(),
                      r.data_ptr(), v.data_ptr(), t.data_ptr(), call.data_ptr(), put.data_ptr(), n),
           "hbsg_blackscholes_arrays")

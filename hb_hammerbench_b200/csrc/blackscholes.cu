@@ -21,16 +21,14 @@
 // on its own (the explicit __f*_rn intrinsics keep nvcc from contracting
 // them); no library math function is called.
 //
-// B200 form: pricing reads 5 floats and writes 2 per option, a few hundred
-// instructions, so the kernel is HBM-bound on both layouts:
+// B200 form: pricing reads 5 floats and writes 2 per option:
 //   - records (the reference's OptionData, 8 floats = 32 bytes, call and put
-//     updated in place): one thread per record loads it as two 16-byte
-//     vectors and stores both back with call and put replaced, so each
-//     record moves as one 32-byte sector each way (64 bytes per option);
+//     updated in place): a record is loaded and stored back whole, one 32-byte
+//     access each way (64 bytes per option). HBM-bound: 10M records 117 -> 96 us,
+//     6.6 TB/s;
 //   - separate arrays (s, strike, r, v, t in; call, put out): 28 bytes per
-//     option, four options per thread as 16-byte vectors.
-// Loads and stores use the streaming (evict-first) cache hint: nothing is
-// reused. Grid-stride loops over one wave of resident CTAs.
+//     option. Bound by the issue rate: 10M options 66 -> 58 us.
+// Each thread prices two options, with packed two-lane arithmetic.
 #include <cuda_runtime.h>
 
 #include "common.cuh"
@@ -39,25 +37,36 @@
 namespace hbsg {
 
 static constexpr int kBsThreads = 256;
-static constexpr int kBsCtasPerSm = 8;
+
+// Two options are priced at a time: every product, sum and fused multiply-add
+// is a packed two-lane instruction (each lane the same IEEE operation), which
+// halves the issue slots of the polynomials; the quotients, reciprocals and
+// square roots, selections and table look-ups stay one per option.
+HBSG_DEV float2 f2(float x) { return make_float2(x, x); }
+HBSG_DEV float2 add2(float2 a, float2 b) { return __fadd2_rn(a, b); }
+HBSG_DEV float2 mul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
+HBSG_DEV float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
+// a - b: b * -1 is exact, so the fused form rounds the difference once, as
+// the subtraction does (signs of zero included)
+HBSG_DEV float2 sub2(float2 a, float2 b) { return fma2(b, f2(-1.0f), a); }
 
 // my_logf (bs_kernel.hpp:33-49)
-HBSG_DEV float bs_logf(float x) {
-  const float diff = __fsub_rn(x, 1.0f);
-  float r = __fmaf_rn(diff, 0.20000000f, -0.25000000f);
-  r = __fmaf_rn(r, diff, 0.33333333f);
-  r = __fmaf_rn(r, diff, -0.50000000f);
-  r = __fmaf_rn(r, diff, 1.00000000f);
-  return __fmul_rn(r, diff);
+HBSG_DEV float2 bs_logf(float2 x) {
+  const float2 diff = add2(x, f2(-1.0f));
+  float2 r = fma2(diff, f2(0.20000000f), f2(-0.25000000f));
+  r = fma2(r, diff, f2(0.33333333f));
+  r = fma2(r, diff, f2(-0.50000000f));
+  r = fma2(r, diff, f2(1.00000000f));
+  return mul2(r, diff);
 }
 
 // expf_0 (bs_kernel.hpp:52-65)
-HBSG_DEV float bs_exp0(float x) {
-  float r = __fmaf_rn(x, 0.0083333338f, 0.04166667f);
-  r = __fmaf_rn(r, x, 0.16666666f);
-  r = __fmaf_rn(r, x, 0.5f);
-  r = __fmaf_rn(r, x, 1.0f);
-  return __fmaf_rn(r, x, 1.0f);
+HBSG_DEV float2 bs_exp0(float2 x) {
+  float2 r = fma2(x, f2(0.0083333338f), f2(0.04166667f));
+  r = fma2(r, x, f2(0.16666666f));
+  r = fma2(r, x, f2(0.5f));
+  r = fma2(r, x, f2(1.0f));
+  return fma2(r, x, f2(1.0f));
 }
 
 // fast_expf (bs_kernel.hpp:69-91), x <= 0, without its loop. The loop
@@ -66,126 +75,170 @@ HBSG_DEV float bs_exp0(float x) {
 // loop runs n = floor(-x) times, leaves x + n (exact, for the same reason) and
 // part1 = the n-fold rounded product, which `pow_tab` (lane k of the warp
 // holds the k-fold product, bs_pow_table) supplies by a shuffle: bit for bit
-// the loop's result. Every lane of the warp must call this together.
-HBSG_DEV float bs_fast_expf(float x, float pow_tab) {
-  const bool zero = x < -15.0f;
-  const int n = (x <= -1.0f && !zero) ? (int)floorf(-x) : 0;  // 0..15
-  float part1 = __shfl_sync(0xffffffffu, pow_tab, n);
-  x = __fadd_rn(x, (float)n);
-  if (x <= -0.5f) {
-    part1 = __fmul_rn(part1, 0.60653066f);
-    x = __fadd_rn(x, 0.5f);
-  }
-  return zero ? 0.0f : __fmul_rn(part1, bs_exp0(x));
+// the loop's result. n is read off 2^23 - x rounded down, whose low mantissa
+// bits it is (0 for -1 < x <= 0; below -15 the result is 0 whatever n is).
+// Every lane of the warp must call this together.
+HBSG_DEV float2 bs_fast_expf(float2 x, float pow_tab) {
+  const float2 t = make_float2(__fadd_rd(8388608.0f, -x.x), __fadd_rd(8388608.0f, -x.y));
+  float2 part1 = make_float2(__shfl_sync(0xffffffffu, pow_tab, __float_as_int(t.x) & 15),
+                             __shfl_sync(0xffffffffu, pow_tab, __float_as_int(t.y) & 15));
+  const float2 y = add2(x, add2(t, f2(-8388608.0f)));
+  // x <= -0.5: one e^-0.5 step (times 1 and plus 0 change nothing otherwise)
+  const bool hx = y.x <= -0.5f, hy = y.y <= -0.5f;
+  part1 = mul2(part1, make_float2(hx ? 0.60653066f : 1.0f, hy ? 0.60653066f : 1.0f));
+  const float2 z = add2(y, make_float2(hx ? 0.5f : 0.0f, hy ? 0.5f : 0.0f));
+  const float2 r = mul2(part1, bs_exp0(z));
+  return make_float2(x.x < -15.0f ? 0.0f : r.x, x.y < -15.0f ? 0.0f : r.y);
 }
 
-// Lane k (< 16) of a warp: e^-1 multiplied into 1.0f k times, each product
-// rounded, as fast_expf's loop forms it.
-HBSG_DEV float bs_pow_table() {
-  const int k = threadIdx.x & 15;
-  float p = 1.0f;
-  for (int i = 0; i < k; ++i) p = __fmul_rn(p, 0.36787945f);
-  return p;
-}
+// The k-fold product of e^-1 for k < 16, each product rounded, as fast_expf's
+// loop forms it (IEEE float products, evaluated by the compiler).
+struct BsPow {
+  float v[16];
+  constexpr BsPow() : v() {
+    float p = 1.0f;
+    for (int k = 0; k < 16; ++k) {
+      v[k] = p;
+      p = p * 0.36787945f;
+    }
+  }
+};
+static __device__ const BsPow g_bs_pow = BsPow();
+
+// Lane k (< 16) of a warp holds the k-fold product.
+HBSG_DEV float bs_pow_table() { return __ldg(&g_bs_pow.v[threadIdx.x & 15]); }
 
 // one lane of dual_CNDF (bs_kernel.hpp:95-160); 1 / (1 + 0.2316419 |x|) as
 // the correctly rounded reciprocal, the same value as the reference's divide
-HBSG_DEV float bs_cndf(float x, float pow_tab) {
-  const bool neg = x < 0.0f;
-  const float xa = fabsf(x);
-  const float e = __fmul_rn(bs_fast_expf(__fmul_rn(__fmul_rn(-0.5f, xa), xa), pow_tab),
-                            0.39894228040143270286f);
-  const float k = __frcp_rn(__fmaf_rn(0.2316419f, xa, 1.0f));
-  float f = __fmaf_rn(k, 1.330274429f, -1.821255978f);
-  f = __fmaf_rn(f, k, 1.781477937f);
-  f = __fmaf_rn(f, k, -0.356563782f);
-  f = __fmaf_rn(f, k, 0.319381530f);
-  f = __fmul_rn(f, k);
-  const float out = __fmaf_rn(-f, e, 1.0f);  // fnmsub.s: -(f * e) + 1
-  return neg ? __fsub_rn(1.0f, out) : out;
+HBSG_DEV float2 bs_cndf(float2 x, float pow_tab) {
+  const float2 xa = make_float2(fabsf(x.x), fabsf(x.y));
+  // -(e^(-x^2/2) * 0.3989...): the sign of the product's constant, so that
+  // fnmsub.s, -(f * e) + 1, is a fused multiply-add of f and -e
+  const float2 ne = mul2(bs_fast_expf(mul2(mul2(f2(-0.5f), xa), xa), pow_tab),
+                         f2(-0.39894228040143270286f));
+  const float2 kd = fma2(f2(0.2316419f), xa, f2(1.0f));
+  const float2 k = make_float2(__frcp_rn(kd.x), __frcp_rn(kd.y));
+  float2 f = fma2(k, f2(1.330274429f), f2(-1.821255978f));
+  f = fma2(f, k, f2(1.781477937f));
+  f = fma2(f, k, f2(-0.356563782f));
+  f = fma2(f, k, f2(0.319381530f));
+  f = mul2(f, k);
+  const float2 out = fma2(f, ne, f2(1.0f));
+  const float2 flip = sub2(f2(1.0f), out);
+  return make_float2(x.x < 0.0f ? flip.x : out.x, x.y < 0.0f ? flip.y : out.y);
 }
 
 // BlkSchlsEqEuroNoDiv_kernel (bs_kernel.hpp:163-198)
-HBSG_DEV void bs_price(float s, float strike, float r, float v, float t, float& call,
-                       float& put, float pow_tab) {
-  const float sqrt_t = __fsqrt_rn(t);
-  const float logv = (s == strike) ? 0.0f : bs_logf(__fdiv_rn(s, strike));
-  float d1 = __fmaf_rn(__fmul_rn(v, v), 0.5f, r);
-  d1 = __fmaf_rn(d1, t, logv);
-  const float den = __fmul_rn(v, sqrt_t);
-  d1 = __fdiv_rn(d1, den);
-  const float d2 = __fsub_rn(d1, den);
-  const float c1 = bs_cndf(d1, pow_tab);
-  const float c2 = bs_cndf(d2, pow_tab);
-  const float fv = __fmul_rn(strike, bs_exp0(__fmul_rn(-r, t)));
-  call = __fsub_rn(__fmul_rn(s, c1), __fmul_rn(fv, c2));
-  put = __fsub_rn(__fmul_rn(fv, __fsub_rn(1.0f, c2)), __fmul_rn(s, __fsub_rn(1.0f, c1)));
+HBSG_DEV void bs_price(float2 s, float2 strike, float2 r, float2 v, float2 t, float2& call,
+                       float2& put, float pow_tab) {
+  const float2 sqrt_t = make_float2(__fsqrt_rn(t.x), __fsqrt_rn(t.y));
+  const float2 lg = bs_logf(make_float2(__fdiv_rn(s.x, strike.x), __fdiv_rn(s.y, strike.y)));
+  const float2 logv = make_float2(s.x == strike.x ? 0.0f : lg.x, s.y == strike.y ? 0.0f : lg.y);
+  float2 d1 = fma2(mul2(v, v), f2(0.5f), r);
+  d1 = fma2(d1, t, logv);
+  const float2 den = mul2(v, sqrt_t);
+  d1 = make_float2(__fdiv_rn(d1.x, den.x), __fdiv_rn(d1.y, den.y));
+  const float2 d2 = sub2(d1, den);
+  const float2 c1 = bs_cndf(d1, pow_tab);
+  const float2 c2 = bs_cndf(d2, pow_tab);
+  const float2 fv = mul2(strike, bs_exp0(mul2(mul2(r, f2(-1.0f)), t)));
+  call = sub2(mul2(s, c1), mul2(fv, c2));
+  put = sub2(mul2(fv, sub2(f2(1.0f), c2)), mul2(s, sub2(f2(1.0f), c1)));
 }
 
-// The grid-stride loops below step whole warps (the loop bound depends on the
-// warp's first index only), because bs_fast_expf shuffles across the warp;
-// lanes past the end price a dummy option and store nothing.
+// Every kernel below prices two options per thread, once: as many CTAs as the
+// options need, so the hardware's scheduler evens out the SMs and a CTA's
+// loads overlap its neighbours' arithmetic and stores. One wave of resident
+// CTAs stepping through the options in a loop measured 107 against 96 us (10M
+// records) and 60 against 58 us (10M in arrays). Lanes past the end price a
+// dummy option and store nothing, because bs_fast_expf shuffles across the
+// warp.
 
-// Records in place, 16-byte aligned: two records per thread per step, all
-// four loads issued before the arithmetic; the whole 32-byte record is stored
-// back (its input fields unchanged), so each record's sector is written whole
-// and never needs a fill from DRAM after the streaming load evicted it.
+// A record as one 32-byte access: its whole DRAM sector in one instruction
+// (as two 16-byte ones 119 instead of 107 us, 10M records). Streamed: nothing
+// is reused.
+struct BsRecord {
+  float f[8];
+};
+template <bool V8>
+HBSG_DEV BsRecord ld_record(const float* p) {
+  BsRecord r;
+  if constexpr (!V8) {  // 16-byte aligned records
+    const float4 x = __ldcs(reinterpret_cast<const float4*>(p));
+    const float4 y = __ldcs(reinterpret_cast<const float4*>(p) + 1);
+    return {{x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w}};
+  }
+  asm volatile(
+      "ld.global.L1::no_allocate.L2::evict_first.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];\n"
+      : "=f"(r.f[0]), "=f"(r.f[1]), "=f"(r.f[2]), "=f"(r.f[3]), "=f"(r.f[4]), "=f"(r.f[5]),
+        "=f"(r.f[6]), "=f"(r.f[7])
+      : "l"(p));
+  return r;
+}
+template <bool V8>
+HBSG_DEV void st_record(float* p, const BsRecord& r) {
+  if constexpr (!V8) {
+    __stcs(reinterpret_cast<float4*>(p), make_float4(r.f[0], r.f[1], r.f[2], r.f[3]));
+    __stcs(reinterpret_cast<float4*>(p) + 1, make_float4(r.f[4], r.f[5], r.f[6], r.f[7]));
+    return;
+  }
+  asm volatile(
+      "st.global.L1::no_allocate.L2::evict_first.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};\n" ::"l"(
+          p),
+      "f"(r.f[0]), "f"(r.f[1]), "f"(r.f[2]), "f"(r.f[3]), "f"(r.f[4]), "f"(r.f[5]), "f"(r.f[6]),
+      "f"(r.f[7])
+      : "memory");
+}
+
+// Records in place, 32-byte (V8) or 16-byte aligned; the whole record is stored back (its
+// input fields unchanged), so its sector is written whole and never needs a
+// fill from DRAM after the streaming load evicted it.
+template <bool V8>
 __global__ void __launch_bounds__(kBsThreads) bs_records_kernel(float* __restrict__ data,
                                                                 long n) {
-  float4* rec = reinterpret_cast<float4*>(data);
   const float pow_tab = bs_pow_table();
-  const long stride = (long)gridDim.x * kBsThreads;
-  const long lane = threadIdx.x & 31;
-  const float4 dummy_a = make_float4(1.f, 1.f, 0.f, 1.f), dummy_b = make_float4(1.f, 0.f, 0.f, 0.f);
-  for (long base = (long)blockIdx.x * kBsThreads + (threadIdx.x & ~31); base < n;
-       base += 2 * stride) {
-    const long i = base + lane, j = i + stride;
-    const bool has0 = i < n, has1 = j < n;
-    float4 a0 = dummy_a, b0 = dummy_b, a1 = dummy_a, b1 = dummy_b;
-    if (has0) {
-      a0 = __ldcs(rec + 2 * i);
-      b0 = __ldcs(rec + 2 * i + 1);
-    }
-    if (has1) {
-      a1 = __ldcs(rec + 2 * j);
-      b1 = __ldcs(rec + 2 * j + 1);
-    }
-    bs_price(a0.x, a0.y, a0.z, a0.w, b0.x, b0.y, b0.z, pow_tab);
-    bs_price(a1.x, a1.y, a1.z, a1.w, b1.x, b1.y, b1.z, pow_tab);
-    if (has0) {
-      __stcs(rec + 2 * i, a0);
-      __stcs(rec + 2 * i + 1, b0);
-    }
-    if (has1) {
-      __stcs(rec + 2 * j, a1);
-      __stcs(rec + 2 * j + 1, b1);
-    }
-  }
+  const long i = (long)blockIdx.x * (2 * kBsThreads) + threadIdx.x, j = i + kBsThreads;
+  BsRecord a = {{1.f, 1.f, 0.f, 1.f, 1.f, 0.f, 0.f, 0.f}}, b = a;
+  if (i < n) a = ld_record<V8>(data + 8 * i);
+  if (j < n) b = ld_record<V8>(data + 8 * j);
+  float2 call, put;
+  bs_price(make_float2(a.f[0], b.f[0]), make_float2(a.f[1], b.f[1]), make_float2(a.f[2], b.f[2]),
+           make_float2(a.f[3], b.f[3]), make_float2(a.f[4], b.f[4]), call, put, pow_tab);
+  a.f[5] = call.x;
+  a.f[6] = put.x;
+  b.f[5] = call.y;
+  b.f[6] = put.y;
+  if (i < n) st_record<V8>(data + 8 * i, a);
+  if (j < n) st_record<V8>(data + 8 * j, b);
 }
 
 // Records at any 4-byte alignment: scalar loads, call and put stored alone.
 __global__ void __launch_bounds__(kBsThreads) bs_records_scalar_kernel(float* __restrict__ data,
                                                                        long n) {
   const float pow_tab = bs_pow_table();
-  const long stride = (long)gridDim.x * kBsThreads;
-  for (long base = (long)blockIdx.x * kBsThreads + (threadIdx.x & ~31); base < n;
-       base += stride) {
-    const long i = base + (threadIdx.x & 31);
-    const bool has = i < n;
-    float* o = data + 8 * (has ? i : 0);
-    float call, put;
-    bs_price(has ? o[0] : 1.f, has ? o[1] : 1.f, has ? o[2] : 0.f, has ? o[3] : 1.f,
-             has ? o[4] : 1.f, call, put, pow_tab);
-    if (has) {
-      o[5] = call;
-      o[6] = put;
-    }
+  const long i = (long)blockIdx.x * (2 * kBsThreads) + threadIdx.x, j = i + kBsThreads;
+  const bool has0 = i < n, has1 = j < n;
+  float* o = data + 8 * (has0 ? i : 0);
+  float* p = data + 8 * (has1 ? j : 0);
+  float2 call, put;
+  bs_price(make_float2(has0 ? o[0] : 1.f, has1 ? p[0] : 1.f),
+           make_float2(has0 ? o[1] : 1.f, has1 ? p[1] : 1.f),
+           make_float2(has0 ? o[2] : 0.f, has1 ? p[2] : 0.f),
+           make_float2(has0 ? o[3] : 1.f, has1 ? p[3] : 1.f),
+           make_float2(has0 ? o[4] : 1.f, has1 ? p[4] : 1.f), call, put, pow_tab);
+  if (has0) {
+    o[5] = call.x;
+    o[6] = put.x;
+  }
+  if (has1) {
+    p[5] = call.y;
+    p[6] = put.y;
   }
 }
 
-// Separate arrays. VEC: all seven arrays 16-byte aligned, four options per
-// thread per step; the last n % 4 options (and every option without VEC) are
-// priced one per thread.
+// Separate arrays. VEC (all seven 8-byte aligned): a thread's two options are
+// consecutive, loaded and stored as 8-byte vectors (the last pair of an odd n
+// holds one option); otherwise they are a CTA's width apart.
 template <bool VEC>
 __global__ void __launch_bounds__(kBsThreads)
     bs_arrays_kernel(const float* __restrict__ s, const float* __restrict__ strike,
@@ -193,72 +246,51 @@ __global__ void __launch_bounds__(kBsThreads)
                      const float* __restrict__ t, float* __restrict__ call,
                      float* __restrict__ put, long n) {
   const float pow_tab = bs_pow_table();
-  const long stride = (long)gridDim.x * kBsThreads;
-  const long wbase = (long)blockIdx.x * kBsThreads + (threadIdx.x & ~31);
-  const long lane = threadIdx.x & 31;
-  long done = 0;
+  float2 C, P;
   if constexpr (VEC) {
-    const long n4 = n / 4;
-    const float4 one = make_float4(1.f, 1.f, 1.f, 1.f);
-    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (long base = wbase; base < n4; base += stride) {
-      const long q = base + lane;
-      const bool has = q < n4;
-      float4 S = one, K = one, R = zero, V = one, T = one;
-      if (has) {
-        S = __ldcs(reinterpret_cast<const float4*>(s) + q);
-        K = __ldcs(reinterpret_cast<const float4*>(strike) + q);
-        R = __ldcs(reinterpret_cast<const float4*>(r) + q);
-        V = __ldcs(reinterpret_cast<const float4*>(v) + q);
-        T = __ldcs(reinterpret_cast<const float4*>(t) + q);
-      }
-      float4 C, P;
-      bs_price(S.x, K.x, R.x, V.x, T.x, C.x, P.x, pow_tab);
-      bs_price(S.y, K.y, R.y, V.y, T.y, C.y, P.y, pow_tab);
-      bs_price(S.z, K.z, R.z, V.z, T.z, C.z, P.z, pow_tab);
-      bs_price(S.w, K.w, R.w, V.w, T.w, C.w, P.w, pow_tab);
-      if (has) {
-        __stcs(reinterpret_cast<float4*>(call) + q, C);
-        __stcs(reinterpret_cast<float4*>(put) + q, P);
-      }
+    const long q = (long)blockIdx.x * kBsThreads + threadIdx.x;
+    const bool both = q < n / 2, one = !both && 2 * q < n;
+    float2 S = f2(1.f), K = f2(1.f), R = f2(0.f), V = f2(1.f), T = f2(1.f);
+    if (both) {
+      S = __ldcs(reinterpret_cast<const float2*>(s) + q);
+      K = __ldcs(reinterpret_cast<const float2*>(strike) + q);
+      R = __ldcs(reinterpret_cast<const float2*>(r) + q);
+      V = __ldcs(reinterpret_cast<const float2*>(v) + q);
+      T = __ldcs(reinterpret_cast<const float2*>(t) + q);
+    } else if (one) {
+      S.x = s[n - 1];
+      K.x = strike[n - 1];
+      R.x = r[n - 1];
+      V.x = v[n - 1];
+      T.x = t[n - 1];
     }
-    done = n4 * 4;
-  }
-  for (long base = done + wbase; base < n; base += stride) {
-    const long i = base + lane;
-    const bool has = i < n;
-    const long ii = has ? i : n - 1;  // lanes past the end read the last option
-    float c, p;
-    bs_price(__ldcs(s + ii), __ldcs(strike + ii), __ldcs(r + ii), __ldcs(v + ii),
-             __ldcs(t + ii), c, p, pow_tab);
-    if (has) {
-      __stcs(call + i, c);
-      __stcs(put + i, p);
+    bs_price(S, K, R, V, T, C, P, pow_tab);
+    if (both) {
+      __stcs(reinterpret_cast<float2*>(call) + q, C);
+      __stcs(reinterpret_cast<float2*>(put) + q, P);
+    } else if (one) {
+      call[n - 1] = C.x;
+      put[n - 1] = P.x;
+    }
+  } else {
+    const long i = (long)blockIdx.x * (2 * kBsThreads) + threadIdx.x, j = i + kBsThreads;
+    const bool has0 = i < n, has1 = j < n;
+    const long ii = has0 ? i : n - 1, jj = has1 ? j : n - 1;  // past the end: the last option
+    bs_price(make_float2(__ldcs(s + ii), __ldcs(s + jj)),
+             make_float2(__ldcs(strike + ii), __ldcs(strike + jj)),
+             make_float2(__ldcs(r + ii), __ldcs(r + jj)),
+             make_float2(__ldcs(v + ii), __ldcs(v + jj)),
+             make_float2(__ldcs(t + ii), __ldcs(t + jj)), C, P, pow_tab);
+    if (has0) {
+      __stcs(call + i, C.x);
+      __stcs(put + i, P.x);
+    }
+    if (has1) {
+      __stcs(call + j, C.y);
+      __stcs(put + j, P.y);
     }
   }
 }
-
-// One wave of resident CTAs (the occupancy of the kernel, looked up once per
-// kernel; at most kBsCtasPerSm per SM), fewer when the work is smaller: the
-// grid-stride loops then give every CTA the same share.
-static int bs_grid(const void* kernel, int* cache, long work, int sms) {
-  int per_sm = __atomic_load_n(cache, __ATOMIC_ACQUIRE);
-  if (per_sm <= 0) {
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kBsThreads, 0) !=
-            cudaSuccess ||
-        per_sm <= 0) {
-      cudaGetLastError();
-      per_sm = 1;
-    }
-    per_sm = per_sm < kBsCtasPerSm ? per_sm : kBsCtasPerSm;
-    __atomic_store_n(cache, per_sm, __ATOMIC_RELEASE);
-  }
-  const long want = (work + kBsThreads - 1) / kBsThreads;
-  const long cap = (long)sms * per_sm;
-  return (int)(want < cap ? (want > 0 ? want : 1) : cap);
-}
-
-static int g_occ_records = 0, g_occ_scalar = 0, g_occ_arrays_vec = 0, g_occ_arrays = 0;
 
 static bool overlaps(const void* a, long abytes, const void* b, long bbytes) {
   const char* x = static_cast<const char*>(a);
@@ -274,18 +306,17 @@ extern "C" int hbsg_blackscholes(hbsg_option* options, int64_t num_option, hbsg_
   if (num_option < 0) return HBSG_ERR_INVALID_ARG;
   if (num_option == 0) return HBSG_OK;
   if (!options) return HBSG_ERR_INVALID_ARG;
-  const int sms = current_device_sms(nullptr);
-  if (sms < 0) return HBSG_ERR_NO_DEVICE;
+  if (current_device_sms(nullptr) < 0) return HBSG_ERR_NO_DEVICE;
   float* data = reinterpret_cast<float*>(options);
   const cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  if ((reinterpret_cast<uintptr_t>(data) & 15) == 0)
-    bs_records_kernel<<<bs_grid((const void*)bs_records_kernel, &g_occ_records,
-                                (num_option + 1) / 2, sms),
-                        kBsThreads, 0, st>>>(data, num_option);
+  const long blocks = (num_option + 2 * kBsThreads - 1) / (2 * kBsThreads);
+  if (blocks > 0x7fffffffL) return HBSG_ERR_UNSUPPORTED;
+  if ((reinterpret_cast<uintptr_t>(data) & 31) == 0)
+    bs_records_kernel<true><<<(unsigned)blocks, kBsThreads, 0, st>>>(data, num_option);
+  else if ((reinterpret_cast<uintptr_t>(data) & 15) == 0)
+    bs_records_kernel<false><<<(unsigned)blocks, kBsThreads, 0, st>>>(data, num_option);
   else
-    bs_records_scalar_kernel<<<bs_grid((const void*)bs_records_scalar_kernel, &g_occ_scalar,
-                                       num_option, sms),
-                               kBsThreads, 0, st>>>(data, num_option);
+    bs_records_scalar_kernel<<<(unsigned)blocks, kBsThreads, 0, st>>>(data, num_option);
   return cudaGetLastError() == cudaSuccess ? HBSG_OK : HBSG_ERR_LAUNCH;
 }
 
@@ -300,18 +331,17 @@ extern "C" int hbsg_blackscholes_arrays(const float* s, const float* strike, con
   if (overlaps(call, nb, put, nb)) return HBSG_ERR_INVALID_ARG;
   for (const float* in : ins)
     if (overlaps(in, nb, call, nb) || overlaps(in, nb, put, nb)) return HBSG_ERR_INVALID_ARG;
-  const int sms = current_device_sms(nullptr);
-  if (sms < 0) return HBSG_ERR_NO_DEVICE;
+  if (current_device_sms(nullptr) < 0) return HBSG_ERR_NO_DEVICE;
   uintptr_t bits = reinterpret_cast<uintptr_t>(call) | reinterpret_cast<uintptr_t>(put);
   for (const float* in : ins) bits |= reinterpret_cast<uintptr_t>(in);
   const cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  if ((bits & 15) == 0)
-    bs_arrays_kernel<true><<<bs_grid((const void*)bs_arrays_kernel<true>, &g_occ_arrays_vec,
-                                     (n + 3) / 4, sms),
-                             kBsThreads, 0, st>>>(s, strike, r, v, t, call, put, n);
+  const long blocks = (n + 2 * kBsThreads - 1) / (2 * kBsThreads);
+  if (blocks > 0x7fffffffL) return HBSG_ERR_UNSUPPORTED;
+  if ((bits & 7) == 0)
+    bs_arrays_kernel<true>
+        <<<(unsigned)blocks, kBsThreads, 0, st>>>(s, strike, r, v, t, call, put, n);
   else
-    bs_arrays_kernel<false><<<bs_grid((const void*)bs_arrays_kernel<false>, &g_occ_arrays, n,
-                                      sms),
-                              kBsThreads, 0, st>>>(s, strike, r, v, t, call, put, n);
+    bs_arrays_kernel<false>
+        <<<(unsigned)blocks, kBsThreads, 0, st>>>(s, strike, r, v, t, call, put, n);
   return cudaGetLastError() == cudaSuccess ? HBSG_OK : HBSG_ERR_LAUNCH;
 }
