@@ -482,7 +482,8 @@ int hbsg_check_device(hbsg_stream_t stream) {
   const int f1 = tc_read_and_clear_device_error();
   const int f2 = grouped_read_and_clear_device_error();
   const int f3 = fused_read_and_clear_device_error();
-  return f1 != HBSG_OK ? f1 : f2 != HBSG_OK ? f2 : f3;
+  const int f4 = jacobi_read_and_clear_device_error();
+  return f1 != HBSG_OK ? f1 : f2 != HBSG_OK ? f2 : f3 != HBSG_OK ? f3 : f4;
 }
 
 int hbsg_debug_timeout_probe(void* workspace, size_t workspace_bytes, hbsg_stream_t stream) {

@@ -116,6 +116,11 @@ bool fused_make_maps(int idx, const float* A, long lda, const float* B, long ldb
 // {box_inner, box_outer}, 128-byte swizzle or none; zeros outside the matrix.
 bool tc_make_f32_map(void* map, const void* base, int inner, int outer, long ld, int box_inner,
                      int box_outer, bool swizzle128);
+// 3-D FP32 map over dense [d2][d1][d0] (d0 a multiple of 4, base 16-byte
+// aligned), no swizzle; zeros outside.
+bool tc_make_f32_map_3d(void* map, const void* base, int d0, int d1, int d2, int box0, int box1,
+                        int box2);
+int jacobi_read_and_clear_device_error();
 // K slices of the automatic schedule for `tiles` output tiles on `slots`
 // concurrent work slots (requested > 0 overrides); shared by both families.
 int tc_slices(long tiles, int K, int slots, int requested, int* kt_per_split);

@@ -25,8 +25,21 @@
 // two edge lanes load the z halo. That issues ~1/3 of the scalar form's
 // instructions per point (the scalar form measured 66 % issue-active at 0.60
 // of the HBM roof on 512^3).
-#include <cuda_runtime.h>
+//
+// Ring form (the vector form's condition, grids of many CTAs): the vector form
+// has one plane's loads in flight per warp and waits for each (5.3 TB/s at 53 %
+// issue-active, DRAM traffic already the ideal 1.05 GB on 512^3). Here a
+// producer warp streams whole (10 rows x 136 z) plane tiles, halos included,
+// through TMA into a ring of kRing planes in shared memory; coordinates
+// outside the grid arrive as zeros, which is the boundary condition. The
+// compute warps march along y reading the ring: x neighbours from the plane's
+// own tile, y neighbours kept in registers. 512^3: 201 -> 164 us (6.55 TB/s, the
+// measured copy bandwidth); 256^3 33.6 -> 28.5 us. Rings of 4-12 planes and
+// slabs of 12-128: 6 planes (33 KB, six CTAs per SM) and slabs of 12 were best
+// (12 planes 171 us, slabs of 32 174 us, of 128 209 us).
+#include <cuda.h>
 
+#include "common.cuh"
 #include "internal.h"
 
 namespace hbsg {
@@ -119,6 +132,151 @@ __global__ void __launch_bounds__(kZ4T * kXT) jacobi_kernel4(float c0f, float c1
   }
 }
 
+// ---- ring form ----------------------------------------------------------------
+static constexpr int kRing = 6;          // plane tiles in flight or in use
+static constexpr int kRingSlab = 12;     // y planes per CTA
+static constexpr int kRingZ = 4 * kZ4T;  // z per CTA
+static constexpr int kTileZ = kRingZ + 8;  // + 4 on either side (16-byte aligned box)
+static constexpr int kTileX = kXT + 2;
+static constexpr int kTileBytes = kTileZ * kTileX * 4;
+static constexpr int kTileStride = (kTileBytes + 127) / 128 * 128;
+static constexpr int kRingThreads = kZ4T * kXT + 32;  // 8 compute warps, 1 producer
+static constexpr int kRingSmem = 128 + kRing * kTileStride + 2 * kRing * 8 + 16;
+static constexpr unsigned long long kRingWaitNs = 4000000000ull;  // bound of every wait
+
+static __device__ int g_jacobi_error = 0;
+
+HBSG_DEV unsigned long long ring_timer() {
+  unsigned long long t;
+  asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+  return t;
+}
+
+// Bounded wait on a barrier phase; false when it expired here or elsewhere in
+// the CTA (every role then leaves its loop).
+HBSG_DEV bool ring_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
+  if (mbar_try_wait(bar, parity)) return true;
+  const unsigned long long t0 = ring_timer();
+  for (uint32_t i = 0;; ++i) {
+    if (mbar_try_wait(bar, parity)) return true;
+    if ((i & 63) == 0) {
+      if (*abort_flag) return false;
+      if (ring_timer() - t0 > kRingWaitNs) {
+        *abort_flag = 1;
+        atomicExch(&g_jacobi_error, (int)HBSG_ERR_DEVICE_TIMEOUT);
+        return false;
+      }
+    }
+  }
+}
+
+__global__ void __launch_bounds__(kRingThreads)
+    jacobi_ring_kernel(const __grid_constant__ CUtensorMap map, float c0f, float c1f,
+                       float* __restrict__ An, int nx, int ny, int nz) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = smem_raw + ((128u - (smem_u32(smem_raw) & 127u)) & 127u);
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem + kRing * kTileStride);
+  uint64_t* empty = full + kRing;
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(empty + kRing);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int zb = blockIdx.x * kRingZ, x0 = blockIdx.y * kXT, y0 = blockIdx.z * kRingSlab;
+  const int y1 = min(ny, y0 + kRingSlab);
+  const int planes = y1 - y0 + 2;  // y0 - 1 .. y1
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < kRing; ++i) {
+      mbar_init(&full[i], 1);
+      mbar_init(&empty[i], kXT);
+    }
+    *abort_flag = 0;
+    fence_barrier_init();
+  }
+  __syncthreads();
+  if (warp == kXT) {
+    // ---- producer: plane p of the slab is y0 - 1 + p ----
+    if (lane == 0) {
+      for (int p = 0; p < planes; ++p) {
+        const int s = p % kRing;
+        if (!ring_wait(&empty[s], ((p / kRing) & 1) ^ 1, abort_flag)) break;
+        mbar_arrive_expect_tx(&full[s], kTileBytes);
+        asm volatile(
+            "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes"
+            " [%0], [%1, {%2, %3, %4}], [%5];\n" ::"r"(smem_u32(smem + s * kTileStride)),
+            "l"(reinterpret_cast<uint64_t>(&map)), "r"(zb - 4), "r"(x0 - 1), "r"(y0 - 1 + p),
+            "r"(smem_u32(&full[s]))
+            : "memory");
+      }
+    }
+  } else {
+    // ---- compute: warp = x row, lane = 4 consecutive z ----
+    const int x = x0 + warp;
+    const int z0 = zb + 4 * lane;
+    const bool live = x < nx && z0 < nz;
+    const float* row = reinterpret_cast<const float*>(smem) + (warp + 1) * kTileZ + 4 + 4 * lane;
+    constexpr int kTileFloats = kTileStride / 4;
+    auto ld4 = [](const float* p) { return *reinterpret_cast<const float4*>(p); };
+    float* out = An + ((long)y0 * nx + (live ? x : 0)) * nz + (live ? z0 : 0);
+    const long sy = (long)nx * nz;
+    float4 ym, cur;
+    // a wait passes when it passed on every lane, so a warp leaves as one
+    bool ok = __all_sync(0xffffffffu, ring_wait(&full[0], 0, abort_flag));
+    if (ok) {
+      ym = ld4(row);
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&empty[0]);
+      ok = __all_sync(0xffffffffu, ring_wait(&full[1], 0, abort_flag));
+    }
+    if (ok) cur = ld4(row + kTileFloats);
+    for (int p = 1; ok && p + 1 < planes; ++p, out += sy) {
+      const int s = p % kRing, sn = (p + 1) % kRing;
+      const float* c_row = row + s * kTileFloats;
+      const float4 xm = ld4(c_row - kTileZ), xp = ld4(c_row + kTileZ);
+      const float up = __shfl_up_sync(0xffffffffu, cur.w, 1);
+      const float dn = __shfl_down_sync(0xffffffffu, cur.x, 1);
+      const float zm0 = lane > 0 ? up : c_row[-1];
+      const float zp3 = lane < kZ4T - 1 ? dn : c_row[4];
+      if (!__all_sync(0xffffffffu, ring_wait(&full[sn], ((p + 1) / kRing) & 1, abort_flag))) break;
+      const float4 yp = ld4(row + sn * kTileFloats);
+      const float xs[4] = {xm.x, xm.y, xm.z, xm.w}, xq[4] = {xp.x, xp.y, xp.z, xp.w};
+      const float ys[4] = {ym.x, ym.y, ym.z, ym.w}, yq[4] = {yp.x, yp.y, yp.z, yp.w};
+      const float c[4] = {cur.x, cur.y, cur.z, cur.w};
+      const float zm[4] = {zm0, cur.x, cur.y, cur.z}, zp[4] = {cur.y, cur.z, cur.w, zp3};
+      float o[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float nb = __fadd_rn(
+            __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(xs[e], xq[e]), ys[e]), yq[e]), zm[e]), zp[e]);
+        o[e] = __fsub_rn(__fmul_rn(c1f, nb), __fmul_rn(c0f, c[e]));
+      }
+      // plane p has been read (its values are in registers) by this warp
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&empty[s]);
+      if (live) __stcs(reinterpret_cast<float4*>(out), make_float4(o[0], o[1], o[2], o[3]));
+      ym = cur;
+      cur = yp;
+    }
+  }
+  // after a bounded abort, copies still in flight get a moment to land
+  if (*abort_flag) {
+    const unsigned long long t0 = ring_timer();
+    while (ring_timer() - t0 < 2000000ull) {
+    }
+  }
+}
+
+static bool ring_map(CUtensorMap* map, const float* A0, int nx, int ny, int nz) {
+  return tc_make_f32_map_3d(map, A0, nz, nx, ny, kTileZ, kTileX, 1);
+}
+
+int jacobi_read_and_clear_device_error() {
+  int v = 0;
+  if (cudaMemcpyFromSymbol(&v, g_jacobi_error, sizeof(int)) != cudaSuccess) return HBSG_ERR_CUDA;
+  if (v != 0) {
+    const int zero = 0;
+    cudaMemcpyToSymbol(g_jacobi_error, &zero, sizeof(int));
+  }
+  return v;
+}
+
 }  // namespace hbsg
 
 using namespace hbsg;
@@ -133,13 +291,34 @@ extern "C" int hbsg_jacobi(int c0, int c1, const float* A0, float* Anext, int nx
   const char* a = reinterpret_cast<const char*>(A0);
   const char* b = reinterpret_cast<const char*>(Anext);
   if (a < b + n * 4 && b < a + n * 4) return HBSG_ERR_INVALID_ARG;
-  if (current_device_sms(nullptr) < 0) return HBSG_ERR_NO_DEVICE;
+  const int sms = current_device_sms(nullptr);
+  if (sms < 0) return HBSG_ERR_NO_DEVICE;
   if ((nz + kZT - 1) / kZT > 0x7fffffff || (nx + kXT - 1) / kXT > 65535 ||
       (ny + kYSlab - 1) / kYSlab > 65535)
     return HBSG_ERR_UNSUPPORTED;
   const cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   const bool vec = (nz & 3) == 0 && ((reinterpret_cast<uintptr_t>(A0) | reinterpret_cast<uintptr_t>(Anext)) & 15) == 0;
-  if (vec) {
+  // The ring form needs a march to stream along: from 17 planes on, where the
+  // vector form starts a second slab and waits for 16 planes one by one
+  // (64^3: 11.7 against 8.5 us), or enough CTAs for every SM. A grid of few
+  // planes stays with the vector form (64 x 8 x 512: 8.0 against 8.6 us with the
+  // tensor map's encoding), and so does one whose z leaves more than half of
+  // the 128-wide tiles outside (512 x 512 x 32: 39.3 against 41.7 us).
+  const long ring_ctas = (long)((nz + kRingZ - 1) / kRingZ) * ((nx + kXT - 1) / kXT) *
+                         ((ny + kRingSlab - 1) / kRingSlab);
+  const bool ring = vec && (ny > kYSlab || ring_ctas >= sms) &&
+                    2L * nz >= ((long)nz + kRingZ - 1) / kRingZ * kRingZ &&
+                    (nx + kXT - 1) / kXT <= 65535 && (ny + kRingSlab - 1) / kRingSlab <= 65535;
+  CUtensorMap map;
+  if (ring && ring_map(&map, A0, nx, ny, nz)) {
+    static uint64_t mask = 0;
+    if (!set_smem_once(reinterpret_cast<const void*>(jacobi_ring_kernel), kRingSmem, &mask))
+      return HBSG_ERR_LAUNCH;
+    const dim3 grid((nz + kRingZ - 1) / kRingZ, (nx + kXT - 1) / kXT,
+                    (ny + kRingSlab - 1) / kRingSlab);
+    jacobi_ring_kernel<<<grid, kRingThreads, kRingSmem, st>>>(map, (float)c0, (float)c1, Anext, nx,
+                                                              ny, nz);
+  } else if (vec) {
     const dim3 grid((nz / 4 + kZ4T - 1) / kZ4T, (nx + kXT - 1) / kXT, (ny + kYSlab - 1) / kYSlab);
     jacobi_kernel4<<<grid, dim3(kZ4T, kXT), 0, st>>>((float)c0, (float)c1, A0, Anext, nx, ny, nz);
   } else {
