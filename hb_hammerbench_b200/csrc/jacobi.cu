@@ -34,7 +34,8 @@
 // outside the grid arrive as zeros, which is the boundary condition. The
 // compute warps march along y reading the ring: x neighbours from the plane's
 // own tile, y neighbours kept in registers. 512^3: 201 -> 164 us (6.55 TB/s, the
-// measured copy bandwidth); 256^3 33.6 -> 28.5 us. Rings of 4-12 planes and
+// measured copy bandwidth), 207 -> 181 us repeated until the power cap holds
+// the clock down; 256^3 33.6 -> 28.5 us. Rings of 4-12 planes and
 // slabs of 12-128: 6 planes (33 KB, six CTAs per SM) and slabs of 12 were best
 // (12 planes 171 us, slabs of 32 174 us, of 128 209 us).
 #include <cuda.h>
@@ -302,12 +303,13 @@ extern "C" int hbsg_jacobi(int c0, int c1, const float* A0, float* Anext, int nx
   // vector form starts a second slab and waits for 16 planes one by one
   // (64^3: 11.7 against 8.5 us), or enough CTAs for every SM. A grid of few
   // planes stays with the vector form (64 x 8 x 512: 8.0 against 8.6 us with the
-  // tensor map's encoding), and so does one whose z leaves more than half of
-  // the 128-wide tiles outside (512 x 512 x 32: 39.3 against 41.7 us).
+  // tensor map's encoding), and so does one whose z leaves more than a quarter
+  // of the 128-wide tiles outside (512 x 512 x 32: 39.3 against 41.7 us; 300 x
+  // 200 x 260: 33.0 against 32.9-35.0 us).
   const long ring_ctas = (long)((nz + kRingZ - 1) / kRingZ) * ((nx + kXT - 1) / kXT) *
                          ((ny + kRingSlab - 1) / kRingSlab);
   const bool ring = vec && (ny > kYSlab || ring_ctas >= sms) &&
-                    2L * nz >= ((long)nz + kRingZ - 1) / kRingZ * kRingZ &&
+                    4L * nz >= 3 * (((long)nz + kRingZ - 1) / kRingZ * kRingZ) &&
                     (nx + kXT - 1) / kXT <= 65535 && (ny + kRingSlab - 1) / kRingSlab <= 65535;
   CUtensorMap map;
   if (ring && ring_map(&map, A0, nx, ny, nz)) {

@@ -1,6 +1,6 @@
 """Jacobi step on grids around the ring form's tiles (128 z, 8 x, slabs of 12
-y) and around the rule that picks it (17 planes, half-filled z tiles, output
-alignment). Bar: bit-exact against the oracle's host_jacobi, nothing written
+y) and around the rule that picks it (17 planes, three-quarter-filled z tiles,
+output alignment). Bar: bit-exact against the oracle's host_jacobi, nothing written
 outside the grid.
 """
 import numpy as np
@@ -12,7 +12,7 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("nx,ny,nz", [
     (8, 24, 128), (8, 17, 128), (8, 16, 128),    # whole tiles; each side of the rule
     (1, 25, 132), (9, 36, 124), (7, 13, 260),    # edge tiles in every direction
-    (17, 37, 64), (3, 40, 60), (10, 18, 516),    # half-filled z tiles, one short of half
+    (17, 37, 96), (3, 40, 92), (10, 18, 516),    # three-quarter-filled z tiles, one quad short
     (5, 100, 4), (2, 19, 254), (40, 12, 1280),   # narrow z, unaligned rows, many CTAs
 ])
 @pytest.mark.parametrize("offset", [0, 4, 1])
