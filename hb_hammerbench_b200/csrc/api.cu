@@ -324,7 +324,8 @@ static int gemm_dispatch(int trans_a, int trans_b, int M, int N, int K, const fl
         ops[n_ops++] = {Ab, lda, M, K, L.Kp, false, nullptr, rowmax};
       if (!(flags & HBSG_FLAG_PRESPLIT_B))
         ops[n_ops++] = {Bb, ldb, N, K, L.Kp, true, ts ? Bp : nullptr, colmax};
-      cudaError_t e = split_operands(ops, n_ops, P, scaled, st);
+      bool after_split = false;
+      cudaError_t e = split_operands(ops, n_ops, P, scaled, st, &after_split);
       if (e != cudaSuccess) return status_from(e);
       if (flags & HBSG_FLAG_SPLIT_ONLY) continue;
       FusedParams fp{};
@@ -344,7 +345,7 @@ static int gemm_dispatch(int trans_a, int trans_b, int M, int N, int K, const fl
       fp.Bparts = ts ? Bp : nullptr;
       fp.Kp = L.Kp;
       e = fused_launch(tc, fp, raster, chunk, sms, 0, st,
-                       reinterpret_cast<float*>(w + L.total));
+                       reinterpret_cast<float*>(w + L.total), after_split);
       if (e != cudaSuccess) return status_from(e);
     }
     return HBSG_OK;
@@ -359,11 +360,12 @@ static int gemm_dispatch(int trans_a, int trans_b, int M, int N, int K, const fl
       ops[n_ops++] = {Ab, lda, M, K, L.Kp, trans_a != 0, Ap, rowmax};
     if (!(flags & HBSG_FLAG_PRESPLIT_B))
       ops[n_ops++] = {Bb, ldb, N, K, L.Kp, trans_b == 0, Bp, colmax};
-    cudaError_t e = split_operands(ops, n_ops, P, scaled, st);
+    bool after_split = false;
+    cudaError_t e = split_operands(ops, n_ops, P, scaled, st, &after_split);
     if (e != cudaSuccess) return status_from(e);
     if (flags & HBSG_FLAG_SPLIT_ONLY) continue;
     e = tc_launch(tc, Ap, Bp, M, N, K, L.Kp, Cb, ldc, rowmax, colmax, raster, chunk, sms, 0, 0, st,
-                  splits, reinterpret_cast<float*>(w + L.total));
+                  splits, reinterpret_cast<float*>(w + L.total), after_split);
     if (e != cudaSuccess) return status_from(e);
   }
   return HBSG_OK;

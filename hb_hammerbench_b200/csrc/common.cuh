@@ -27,6 +27,15 @@ HBSG_DEV void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
 }
 
+// ---- programmatic dependent launch ------------------------------------------
+// A kernel launched with launch_after(..., true) may start while the kernel
+// before it in the stream still runs, once every CTA of that one has called
+// grid_dep_trigger (or exited). grid_dep_wait returns when that kernel has
+// completed and its writes are visible; nothing it writes may be touched
+// before. Both do nothing in an ordinary launch.
+HBSG_DEV void grid_dep_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
+HBSG_DEV void grid_dep_trigger() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
+
 HBSG_DEV uint32_t smem_u32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }

@@ -44,8 +44,10 @@ struct SplitOperand {
   void* parts;
   uint32_t* mx;
 };
+// *launched: the last thing it put on the stream was a split kernel (see
+// launch_after).
 cudaError_t split_operands(const SplitOperand* ops, int n, int parts, bool scaled,
-                           cudaStream_t st);
+                           cudaStream_t st, bool* launched);
 int tc_num_tiles();
 bool tc_tile_info(int idx, hbsg_tile_info* out);
 int tc_tile_parts(int idx);
@@ -57,7 +59,7 @@ cudaError_t tc_launch(int idx, const void* Ap, const void* Bp, int M, int N, int
                       float* C, long ldc, const uint32_t* rowmax, const uint32_t* colmax,
                       int raster, int chunk_k, int sms, int debug_skip_loads,
                       unsigned long long wait_limit_ns, cudaStream_t st, int splits = 1,
-                      float* partial = nullptr);
+                      float* partial = nullptr, bool after_split = false);
 int tc_pick_splits(int idx, int M, int N, int K, int requested, int sms, int* kt_per_split);
 int ffma_pick_splits(int tile_idx, int M, int N, int K, int batch, int requested, int sms);
 // C[b] = sum over s of partial[b][s] (fixed order), partial rows of N floats.
@@ -100,7 +102,8 @@ int fused_tile_slots(int idx, int sms);  // concurrent work units (clusters or C
 int fused_pick_splits(int idx, int M, int N, int K, int requested, int sms, int* kt_per_split);
 // C = A*B on fused entry idx; partial: [splits][M][N] FP32 when p.splits > 1.
 cudaError_t fused_launch(int idx, FusedParams p, int raster, int chunk_k, int sms,
-                         unsigned long long wait_limit_ns, cudaStream_t st, float* partial);
+                         unsigned long long wait_limit_ns, cudaStream_t st, float* partial,
+                         bool after_split);
 int fused_read_and_clear_device_error();
 int fused_l2_ahead();
 // Measured SM cycles one CTA of fused entry idx spends per k-tile (the
@@ -129,6 +132,27 @@ int tc_slices(long tiles, int K, int slots, int requested, int* kt_per_split);
 size_t gemm_workspace_exact(int trans_a, int trans_b, int m, int n, int k, const float* a,
                             long lda, const float* b, long ldb, int variant,
                             const hbsg_config* cfg);
+
+// Launches `kernel`; with `early` as a programmatic dependent of the kernel
+// before it in the stream (common.cuh): its launch and its set-up (barriers,
+// tensor memory, loads that do not depend on that kernel) overlap that
+// kernel's tail. Only set where this library launched that kernel just before
+// in the same call, so that whatever ran earlier is known to be complete.
+template <class... Params, class... Args>
+cudaError_t launch_after(void (*kernel)(Params...), unsigned grid, unsigned block, int smem,
+                         cudaStream_t st, bool early, const Args&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid, 1, 1);
+  cfg.blockDim = dim3(block, 1, 1);
+  cfg.dynamicSmemBytes = (size_t)smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = early ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, Params(args)...);
+}
 
 // ---- device state -------------------------------------------------------------
 // Device ordinals the per-device tables cover (one bit each in a uint64_t).

@@ -160,6 +160,8 @@ HBSG_DEV void split_job(const SplitJob& j, unsigned block, float (*tile)[65]) {
 template <int P, bool SCALED>
 __global__ void __launch_bounds__(kSplitThreads) split_kernel(const __grid_constant__ SplitJobs jobs) {
   __shared__ float tile[64][65];
+  grid_dep_trigger();  // the next split launch or the product may set itself up
+  grid_dep_wait();     // second launch: the first one's maxima
   if (blockIdx.x < jobs.first1) split_job<P, SCALED>(jobs.job[0], blockIdx.x, tile);
   else split_job<P, SCALED>(jobs.job[1], blockIdx.x - jobs.first1, tile);
 }
@@ -175,7 +177,8 @@ static long blocks_of(const SplitJob& j) {
   }
 }
 
-static cudaError_t launch_jobs(SplitJob* job, int n, int parts, bool scaled, cudaStream_t st) {
+static cudaError_t launch_jobs(SplitJob* job, int n, int parts, bool scaled, cudaStream_t st,
+                               bool* launched) {
   // grids are one-dimensional: at most 2^31 - 1 blocks, each launch takes as
   // many jobs as fit (one operand alone always does: its elements are
   // addressable by 32-bit row and k)
@@ -185,16 +188,13 @@ static cudaError_t launch_jobs(SplitJob* job, int n, int parts, bool scaled, cud
   auto flush = [&]() -> cudaError_t {
     if (total == 0) return cudaSuccess;
     const unsigned grid = (unsigned)total;
-    if (parts == 3) {
-      if (scaled) split_kernel<3, true><<<grid, kSplitThreads, 0, st>>>(jobs);
-      else split_kernel<3, false><<<grid, kSplitThreads, 0, st>>>(jobs);
-    } else {
-      if (scaled) split_kernel<2, true><<<grid, kSplitThreads, 0, st>>>(jobs);
-      else split_kernel<2, false><<<grid, kSplitThreads, 0, st>>>(jobs);
-    }
+    void (*k)(SplitJobs) = parts == 3 ? (scaled ? split_kernel<3, true> : split_kernel<3, false>)
+                                      : (scaled ? split_kernel<2, true> : split_kernel<2, false>);
+    const cudaError_t e = launch_after(k, grid, kSplitThreads, 0, st, *launched, jobs);
+    *launched = e == cudaSuccess;
     total = 0;
     taken = 0;
-    return cudaGetLastError();
+    return e;
   };
   for (int i = 0; i < n; ++i) {
     const long b = blocks_of(job[i]);
@@ -214,7 +214,8 @@ static cudaError_t launch_jobs(SplitJob* job, int n, int parts, bool scaled, cud
 }
 
 cudaError_t split_operands(const SplitOperand* ops, int n, int parts, bool scaled,
-                           cudaStream_t st) {
+                           cudaStream_t st, bool* launched) {
+  *launched = false;
   SplitJob first[2], second[2];
   int n1 = 0, n2 = 0;
   for (int i = 0; i < n; ++i) {
@@ -236,8 +237,8 @@ cudaError_t split_operands(const SplitOperand* ops, int n, int parts, bool scale
       if (o.parts) second[n2++] = j;
     }
   }
-  const cudaError_t e = launch_jobs(first, n1, parts, scaled, st);
-  return e != cudaSuccess ? e : launch_jobs(second, n2, parts, scaled, st);
+  const cudaError_t e = launch_jobs(first, n1, parts, scaled, st, launched);
+  return e != cudaSuccess ? e : launch_jobs(second, n2, parts, scaled, st, launched);
 }
 
 }  // namespace hbsg

@@ -101,18 +101,18 @@ static const void* fused_kernel_ptr(bool scaled) {
 
 template <int P, int BN, int STAGES, int SSTAGES>
 static cudaError_t launch_fused(const CUtensorMap& a, const CUtensorMap& b, const FusedParams& p,
-                                const TcRun& run, int grid, cudaStream_t st, bool scaled) {
+                                const TcRun& run, int grid, cudaStream_t st, bool scaled,
+                                bool after_split) {
   using S = TcFusedShape<P, BN, STAGES, SSTAGES>;
   const void* k = fused_kernel_ptr<P, BN, STAGES, SSTAGES>(scaled);
   static uint64_t masks[2] = {0, 0};
   if (!set_smem_once(k, S::kSmemBytes, &masks[scaled ? 1 : 0])) return cudaErrorInvalidValue;
   static int regs_ok[2] = {0, 0};
   if (!fused_regs_ok(k, &regs_ok[scaled ? 1 : 0])) return cudaErrorInvalidConfiguration;
-  if (scaled)
-    tc_fused_kernel<P, BN, STAGES, SSTAGES, true><<<grid, kFusedThreads, S::kSmemBytes, st>>>(a, b, p, run);
-  else
-    tc_fused_kernel<P, BN, STAGES, SSTAGES, false><<<grid, kFusedThreads, S::kSmemBytes, st>>>(a, b, p, run);
-  return cudaGetLastError();
+  auto kernel = scaled ? tc_fused_kernel<P, BN, STAGES, SSTAGES, true>
+                       : tc_fused_kernel<P, BN, STAGES, SSTAGES, false>;
+  return launch_after(kernel, (unsigned)grid, kFusedThreads, S::kSmemBytes, st, after_split, a, b, p,
+                      run);
 }
 
 template <int P, int BN, int STAGES, int SSTAGES>
@@ -135,7 +135,7 @@ static const void* fused_ts_kernel_ptr(bool scaled) {
 template <int P, int BN, int SA, int SB, int TSTAGES, int KS>
 static cudaError_t launch_fused_ts(const CUtensorMap& a, const CUtensorMap& b,
                                    const FusedParams& p, const TcRun& run, int grid,
-                                   cudaStream_t st, bool scaled) {
+                                   cudaStream_t st, bool scaled, bool after_split) {
   using S = TcTsShape<P, BN, SA, SB, TSTAGES, KS>;
   const void* k = fused_ts_kernel_ptr<P, BN, SA, SB, TSTAGES, KS>(scaled);
   static uint64_t masks[2] = {0, 0};
@@ -144,11 +144,10 @@ static cudaError_t launch_fused_ts(const CUtensorMap& a, const CUtensorMap& b,
     static int regs_ok[2] = {0, 0};
     if (!fused_regs_ok(k, &regs_ok[scaled ? 1 : 0])) return cudaErrorInvalidConfiguration;
   }
-  if (scaled)
-    tc_fused_ts_kernel<P, BN, SA, SB, TSTAGES, KS, true><<<grid, kTsThreads, S::kSmemBytes, st>>>(a, b, p, run);
-  else
-    tc_fused_ts_kernel<P, BN, SA, SB, TSTAGES, KS, false><<<grid, kTsThreads, S::kSmemBytes, st>>>(a, b, p, run);
-  return cudaGetLastError();
+  auto kernel = scaled ? tc_fused_ts_kernel<P, BN, SA, SB, TSTAGES, KS, true>
+                       : tc_fused_ts_kernel<P, BN, SA, SB, TSTAGES, KS, false>;
+  return launch_after(kernel, (unsigned)grid, kTsThreads, S::kSmemBytes, st, after_split, a, b, p,
+                      run);
 }
 
 // Resident CTAs of an A-in-TMEM kernel (0 if unknown).
@@ -178,7 +177,7 @@ struct FusedEntry {
   int bm;       // output rows per tile
   int threads;  // per CTA
   cudaError_t (*launch)(const CUtensorMap&, const CUtensorMap&, const FusedParams&, const TcRun&,
-                        int, cudaStream_t, bool);
+                        int, cudaStream_t, bool scaled, bool after_split);
   int (*slots)(bool);  // concurrently resident work units: clusters of two, or CTAs (ts)
 };
 
@@ -261,7 +260,8 @@ bool fused_make_maps(int idx, const float* A, long lda, const float* B, long ldb
 }
 
 cudaError_t fused_launch(int idx, FusedParams p, int raster, int chunk_k, int sms,
-                         unsigned long long wait_limit_ns, cudaStream_t st, float* partial) {
+                         unsigned long long wait_limit_ns, cudaStream_t st, float* partial,
+                         bool after_split) {
   const FusedEntry& e = kFused[idx];
   CUtensorMap ma, mb;
   if (p.K > 0) {
@@ -304,7 +304,8 @@ cudaError_t fused_launch(int idx, FusedParams p, int raster, int chunk_k, int sm
   int resident = e.slots(scaled);
   if (resident <= 0 || resident > cap) resident = cap;
   const long units = std::max<long>(1, std::min<long>(items, resident));
-  cudaError_t err = e.launch(ma, mb, p, run, (int)(e.ts ? units : 2 * units), st, scaled);
+  cudaError_t err = e.launch(ma, mb, p, run, (int)(e.ts ? units : 2 * units), st, scaled,
+                             after_split);
   if (err != cudaSuccess || p.splits == 1) return err;
   return splitk_reduce(partial, C, p.M, p.N, ldc, 0, p.splits, 1, sms, st);
 }

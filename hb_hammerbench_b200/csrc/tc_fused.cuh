@@ -366,6 +366,7 @@ __device__ __forceinline__ void tc_fused_body(const Tiles& tiles, const TcRun& r
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   const unsigned long long lim = run.wait_limit_ns;
+  grid_dep_wait();  // the split pass's parts and maxima (set-up above overlaps its tail)
 
   // Each role's code sits inside the branch that set its register count, so
   // the compiler allocates the epilogue's sums under the larger limit.

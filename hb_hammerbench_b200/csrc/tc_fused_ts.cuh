@@ -194,6 +194,7 @@ __device__ __forceinline__ void tc_fused_ts_body(const Tiles& tiles, const TcRun
     // zeros); B: the k-tile's 32 k of BN rows of every part
     if (lane == 0) {
       const bool a_role = warp == 0;
+      if (!a_role) grid_dep_wait();  // B's parts; A's loads and conversion start without them
       uint32_t it = 0;
       bool ok = true;
       for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x) {
@@ -320,6 +321,7 @@ __device__ __forceinline__ void tc_fused_ts_body(const Tiles& tiles, const TcRun
     int ex = 0;
     uint32_t it = 0;
     bool ok = true;
+    if constexpr (SCALED) grid_dep_wait();  // row maxima
     for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x) {
       const TileWork w = tiles.get(t);
       if constexpr (SCALED) {
@@ -388,6 +390,7 @@ __device__ __forceinline__ void tc_fused_ts_body(const Tiles& tiles, const TcRun
   } else if (warp >= 12) {
     // ---------------- epilogue (warps 12-15) ----------------
     if constexpr (kSplitRegs) regs_inc<kTsRegsHigh>();
+    grid_dep_wait();  // column maxima; outputs follow everything before this call
     const int q = warp & 3;
     uint32_t ch = 0;
     bool ok = true;

@@ -192,12 +192,13 @@ struct TcEntry {
   int pair;  // 1: CTA-pair kernel, 256-row tiles
   int smem;
   cudaError_t (*launch)(const CUtensorMap&, const CUtensorMap&, const TcParams&, const TcRun&,
-                        int grid, cudaStream_t, bool scaled);
+                        int grid, cudaStream_t, bool scaled, bool after_split);
 };
 
 template <int P, int BN, int STAGES>
 static cudaError_t launch_tc(const CUtensorMap& a, const CUtensorMap& b, const TcParams& p,
-                             const TcRun& run, int grid, cudaStream_t st, bool scaled) {
+                             const TcRun& run, int grid, cudaStream_t st, bool scaled,
+                             bool after_split) {
   using S = TcShape<P, BN, STAGES>;
   auto k0 = tc_gemm_kernel<P, BN, STAGES, false>;
   auto k1 = tc_gemm_kernel<P, BN, STAGES, true>;
@@ -205,8 +206,7 @@ static cudaError_t launch_tc(const CUtensorMap& a, const CUtensorMap& b, const T
   static uint64_t m0 = 0, m1 = 0;
   if (!set_smem_once(reinterpret_cast<const void*>(k), S::kSmemBytes, scaled ? &m1 : &m0))
     return cudaErrorInvalidValue;
-  k<<<grid, S::kThreads, S::kSmemBytes, st>>>(a, b, p, run);
-  return cudaGetLastError();
+  return launch_after(k, (unsigned)grid, S::kThreads, S::kSmemBytes, st, after_split, a, b, p, run);
 }
 
 #define HBSG_TC_ENTRY(P, BN, ST) \
@@ -215,7 +215,8 @@ static cudaError_t launch_tc(const CUtensorMap& a, const CUtensorMap& b, const T
 // Ordered by parts: entries with parts == 3 serve BF16X6, parts == 2 BF16X3.
 template <int P, int BN, int STAGES>
 static cudaError_t launch_tc_pair(const CUtensorMap& a, const CUtensorMap& b, const TcParams& p,
-                                  const TcRun& run, int grid, cudaStream_t st, bool scaled) {
+                                  const TcRun& run, int grid, cudaStream_t st, bool scaled,
+                             bool after_split) {
   using S = TcPairShape<P, BN, STAGES>;
   auto k0 = tc_pair_kernel<P, BN, STAGES, false>;
   auto k1 = tc_pair_kernel<P, BN, STAGES, true>;
@@ -223,8 +224,7 @@ static cudaError_t launch_tc_pair(const CUtensorMap& a, const CUtensorMap& b, co
   static uint64_t m0 = 0, m1 = 0;
   if (!set_smem_once(reinterpret_cast<const void*>(k), S::kSmemBytes, scaled ? &m1 : &m0))
     return cudaErrorInvalidValue;
-  k<<<grid, 320, S::kSmemBytes, st>>>(a, b, p, run);
-  return cudaGetLastError();
+  return launch_after(k, (unsigned)grid, 320, S::kSmemBytes, st, after_split, a, b, p, run);
 }
 #define HBSG_TC_PAIR_ENTRY(P, BN, ST) \
   TcEntry { P, BN, ST, 1, TcPairShape<P, BN, ST>::kSmemBytes, &launch_tc_pair<P, BN, ST> }
@@ -375,7 +375,7 @@ cudaError_t tc_launch(int idx, const void* Ap, const void* Bp, int M, int N, int
                       float* C, long ldc, const uint32_t* rowmax, const uint32_t* colmax,
                       int raster, int chunk_k, int sms, int debug_skip_loads,
                       unsigned long long wait_limit_ns, cudaStream_t st, int splits,
-                      float* partial) {
+                      float* partial, bool after_split) {
   const TcEntry& e = kTcTiles[idx];
   CUtensorMap ma, mb;
   if (!tc_make_parts_map_impl(&ma, Ap, e.parts, M, Kp, kBM)) return cudaErrorInvalidValue;
@@ -417,7 +417,7 @@ cudaError_t tc_launch(int idx, const void* Ap, const void* Bp, int M, int N, int
   } else {
     grid = (int)(items < sms ? items : sms);
   }
-  cudaError_t err = e.launch(ma, mb, p, run, grid, st, rowmax != nullptr);
+  cudaError_t err = e.launch(ma, mb, p, run, grid, st, rowmax != nullptr, after_split);
   if (err != cudaSuccess || p.splits == 1) return err;
   return splitk_reduce(partial, C, M, N, ldc, 0, p.splits, 1, sms, st);
 }

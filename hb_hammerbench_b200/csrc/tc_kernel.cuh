@@ -437,6 +437,7 @@ __device__ __forceinline__ void tc_body(const Tiles& tiles, const TcRun& run) {
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   const unsigned long long lim = run.wait_limit_ns;
+  grid_dep_wait();  // the split pass's parts and maxima (set-up above overlaps its tail)
 
   // Next entry of the tile queue for a consumer (the MMA issuer, or lane 0 of
   // an epilogue warp): {tile or -1, k-tiles, MMA width, valid rows}; false on

@@ -120,6 +120,7 @@ __device__ __forceinline__ void tc_pair_body(const Tiles& tiles, const TcRun& ru
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   const unsigned long long lim = run.wait_limit_ns;
+  grid_dep_wait();  // the split pass's parts and maxima (set-up above overlaps its tail)
 
   if (warp == 0) {
     // ---------------- TMA producer (both CTAs) ----------------
