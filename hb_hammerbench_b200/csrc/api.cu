@@ -109,17 +109,114 @@ struct TcChoice {
   int splits, kts;
 };
 
-// Automatic choice between the split-pass tiles and the fused-split tiles by
-// estimated time on this shape:
-//   split pass: its HBM traffic (read FP32, write the parts) plus the product
-//     at the tile's score times the tensor-core rate;
-//   fused: waves x k-tiles per work item x the measured per-k-tile cycles of
-//     the tile, at least the FP32 operands' HBM time, plus the split-K reduce.
-// The fused form is taken only when it is estimated >10 % faster. It wins
-// where the split pass is a large share: small outputs with long K (all of
-// 256 x 256 x 1048576's time is operand traffic) and tall, narrow products.
+// ---- automatic split-BF16 schedule ----
+// Estimated microseconds of a call on a tile with s K slices:
+//   fixed                         launches, set-up, first loads, last stores
+// + split  x operand bytes of the tile's split pass (read FP32, write the
+//            parts) / 6 TB/s
+// + wave   x rounds of the concurrent slots (an epilogue each)
+// + ktile  x rounds x k-tiles per slice
+// + s > 1: reduce x partial bytes written and read / 10 TB/s, + sliced
+// The coefficients are a least-squares fit, tile by tile, to GPU times of 118
+// shapes (M, N, K of 128-8192 and long-K and tall ones, every tile, 1-148
+// slices; rms error 4-9 %). Taking the tile and slices of least estimate runs
+// those shapes within 0.4 % of the best measured choice in the geometric mean
+// (13 % at worst); the rule before it, which scored tiles by their last wave
+// and sliced K only into slices of 16 k-tiles for outputs under half the SMs,
+// within 20 % (6.4x at worst: 224 x 160 x 3136 in 6 products 44 against 17 us).
+// `sliced` holds 3 us beyond the fit for the reduction's launch, which a
+// host-bound caller pays in full.
+struct TileCost {
+  double fixed, split, wave, ktile, reduce, sliced;
+};
+static const TileCost kTcCost[] = {
+    {5.6, 1.28, 5.13, 0.708, 1.38, 3.0},  // 6 products, 128 x 256
+    {6.0, 1.09, 1.33, 0.507, 0.51, 4.5},  // 128 x 128
+    {5.4, 1.01, 0.73, 0.452, 0.00, 4.9},  // 128 x 64
+    {4.7, 1.20, 4.96, 0.413, 0.60, 4.1},  // 3 products, 128 x 256
+    {5.2, 1.07, 1.49, 0.311, 0.29, 4.7},  // 128 x 128
+    {4.9, 0.98, 0.77, 0.293, 0.00, 5.0},  // 128 x 64
+    {6.1, 1.20, 2.39, 0.608, 0.97, 3.6},  // 6 products, 128 x 192
+    {4.9, 1.11, 2.69, 0.352, 0.51, 4.4},  // 3 products, 128 x 192
+    {5.3, 1.23, 4.79, 0.863, 0.57, 3.6},  // 6 products, pair 256 x 256
+    {4.9, 1.20, 5.12, 0.417, 0.47, 4.2},  // 3 products, pair 256 x 256
+};
+static const TileCost kFusedCost[] = {
+    {8.8, 0.00, 1.59, 1.394, 1.65, 3.0},  // 6 products, pair 256 x 256
+    {8.7, 0.00, 1.34, 1.192, 1.34, 3.0},  // 3 products
+    {7.3, 0.00, 0.00, 1.095, 1.06, 3.0},  // 6 products, pair 256 x 64
+    {6.7, 0.00, 0.00, 0.992, 0.71, 3.0},  // 3 products
+    {5.2, 1.10, 1.18, 0.364, 0.62, 5.1},  // 6 products, A in TMEM, 128 x 64
+    {5.1, 1.12, 0.96, 0.257, 0.30, 5.1},  // 3 products
+    {5.3, 1.07, 3.23, 0.557, 0.79, 5.1},  // 6 products, A in TMEM, 128 x 128
+    {5.1, 1.09, 3.24, 0.352, 0.63, 5.2},  // 3 products
+};
+
+static double tile_us(const TileCost& c, double split_bytes, long tiles, int slots, int KT, int s,
+                      double mn) {
+  const int per = (KT + s - 1) / s;
+  const int slices = (KT + per - 1) / per;
+  const double waves = (double)((tiles * slices + slots - 1) / slots);
+  double t = c.fixed + c.split * split_bytes / 6e6 + c.wave * waves + c.ktile * waves * per;
+  if (slices > 1) t += c.reduce * slices * mn * 8.0 / 1e7 + c.sliced;
+  return t;
+}
+
+// Slice counts tried when the caller names none: each at least 8 k-tiles, and
+// no more than about two rounds of the slots.
+static const int kSliceCounts[] = {1, 2, 3, 4, 6, 8, 12, 16, 24, 37, 48, 74, 111, 148};
+
 static void tc_pick_auto(int M, int N, int K, int variant, int sms, int req, bool fusable,
                          TcChoice* ch) {
+  const int P = parts_of(variant);
+  const int KT = K > 0 ? (K + 31) / 32 : 1;
+  const double mk = (double)M * K, kn = (double)K * N, mn = (double)M * N;
+  const double per_elem = 4.0 + 2.0 * P;
+  const bool scaled = scaled_of(variant);
+  double best = 0.0;
+  int best_s = 1;
+  bool have = false;
+  auto consider = [&](bool fused, int idx, const TileCost& c, int bm, int bn, int slots,
+                      double split_bytes) {
+    const long tiles = (long)((M + bm - 1) / bm) * ((N + bn - 1) / bn);
+    for (int s : kSliceCounts) {
+      if (req > 0) s = req;
+      if (req <= 0 && s > 1 && (KT / s < 8 || tiles * s * 5 > 11L * slots)) break;
+      const double t = tile_us(c, split_bytes, tiles, slots, KT, s < KT ? s : KT, mn);
+      if (!have || t < best) {
+        have = true;
+        best = t;
+        best_s = s;
+        ch->fused = fused;
+        ch->idx = idx;
+      }
+      if (req > 0) break;
+    }
+  };
+  for (int i = 0; i < tc_num_tiles(); ++i) {
+    if (tc_tile_parts(i) != P) continue;
+    const bool pair = tc_tile_pair(i) != 0;
+    // scaled: the rows' maxima ride on their split, the columns are read again
+    consider(false, i, kTcCost[i], pair ? 256 : 128, tc_tile_bn(i), pair ? sms / 2 : sms,
+             (mk + kn) * per_elem + (scaled ? kn * 4.0 : 0.0));
+  }
+  if (fusable && K > 0) {
+    for (int f = 0; f < fused_num_tiles(); ++f) {
+      if (fused_tile_parts(f) != P) continue;
+      const double bytes = (fused_tile_ts(f) ? kn * per_elem : 0.0) + (scaled ? (mk + kn) * 4.0 : 0.0);
+      consider(true, f, kFusedCost[f], fused_tile_bm(f), fused_tile_bn(f),
+               fused_tile_slots(f, sms), bytes);
+    }
+  }
+  ch->splits = ch->fused ? fused_pick_splits(ch->idx, M, N, K, best_s, sms, &ch->kts)
+                         : tc_pick_splits(ch->idx, M, N, K, best_s, sms, &ch->kts);
+}
+
+// A schedule with fewer K slices, so less workspace: run where the automatic
+// choice's partials do not fit the caller's buffer, and the measure of which
+// problems the allocation-free entry point takes. Tiles by their score
+// (split-pass tiles) or by waves of measured k-tile cycles (fused ones).
+static void tc_pick_compact(int M, int N, int K, int variant, int sms, bool fusable, TcChoice* ch) {
   constexpr double kRate = 1.6e15;  // BF16 MMA flop/s of a well-fed tile
   constexpr double kHbm = 6.0e12;   // bytes/s of the split and product passes
   constexpr double kClock = 1.5e9;  // SM clock under load
@@ -130,7 +227,8 @@ static void tc_pick_auto(int M, int N, int K, int variant, int sms, int req, boo
   const double maxima = scaled_of(variant) ? opnds * 4.0 / kHbm : 0.0;
   double score = 0.0;
   ch->fused = false;
-  ch->idx = tc_pick_tile(M, N, K, P, sms, req, &score);
+  ch->idx = tc_pick_tile(M, N, K, P, sms, 0, &score);
+  ch->splits = tc_pick_splits(ch->idx, M, N, K, 0, sms, &ch->kts);
   if (!fusable || K <= 0 || score <= 0.0) return;
   const double t_split = opnds * (4.0 + 2.0 * P) / (0.9 * kHbm) + 6e-6;
   const double t_unfused = t_split + flops / (kRate * score) + maxima;
@@ -143,7 +241,7 @@ static void tc_pick_auto(int M, int N, int K, int variant, int sms, int req, boo
     const int slots = fused_tile_slots(f, sms);
     const long tiles = (long)((M + bm - 1) / bm) * ((N + bn - 1) / bn);
     int kts = 0;
-    const int s = fused_pick_splits(f, M, N, K, req, sms, &kts);
+    const int s = fused_pick_splits(f, M, N, K, 0, sms, &kts);
     const long waves = (tiles * s + slots - 1) / slots;
     const double t_conv = (double)waves * kts * fused_ktile_cycles(f) / kClock;
     const double t_mem = opnds * 4.0 / kHbm;
@@ -164,6 +262,8 @@ static void tc_pick_auto(int M, int N, int K, int variant, int sms, int req, boo
     ch->fused = true;
     ch->idx = best_idx;
   }
+  ch->splits = ch->fused ? fused_pick_splits(ch->idx, M, N, K, 0, sms, &ch->kts)
+                         : tc_pick_splits(ch->idx, M, N, K, 0, sms, &ch->kts);
 }
 
 // Tensor-core tile and K-slice count for a split-BF16 problem (shared by the
@@ -190,6 +290,7 @@ static bool tc_schedule(int M, int N, int K, int variant, const hbsg_config* cfg
     }
   } else {
     tc_pick_auto(M, N, K, variant, sms, req, !transposed && fusable, ch);
+    return true;
   }
   ch->splits = ch->fused ? fused_pick_splits(ch->idx, M, N, K, req, sms, &ch->kts)
                          : tc_pick_splits(ch->idx, M, N, K, req, sms, &ch->kts);
@@ -233,6 +334,18 @@ size_t gemm_workspace_exact(int trans_a, int trans_b, int m, int n, int k, const
   if (m <= 0 || n <= 0 || k < 0 || !variant_valid(variant)) return 0;
   return workspace_needed(m, n, k, 1, variant, cfg, trans_a || trans_b,
                           operands_fusable(k, a, lda, 0, b, ldb, 0) ? 1 : 0);
+}
+
+size_t gemm_compact_workspace(int trans_a, int trans_b, int m, int n, int k, const float* a,
+                              long lda, const float* b, long ldb, int variant) {
+  const int sms = current_device_sms(nullptr);
+  if (m <= 0 || n <= 0 || k < 0 || !variant_valid(variant) || sms < 0) return 0;
+  const bool fusable = !(trans_a || trans_b) && operands_fusable(k, a, lda, 0, b, ldb, 0);
+  TcChoice ch;
+  tc_pick_compact(m, n, k, variant, sms, fusable, &ch);
+  return (ch.fused ? fused_layout(m, n, k, variant, fused_tile_ts(ch.idx))
+                   : split_layout(m, n, k, variant)).total +
+         (ch.splits > 1 ? align256((size_t)ch.splits * m * n * 4) : 0);
 }
 
 // Core dispatcher for one (possibly batched) GEMM.
@@ -294,13 +407,27 @@ static int gemm_dispatch(int trans_a, int trans_b, int M, int N, int K, const fl
   const bool fusable = operands_fusable(K, A, lda, strideA, B, ldb, strideB);
   if (!tc_schedule(M, N, K, variant, cfg, sms, trans_a || trans_b, fusable, &ch))
     return HBSG_ERR_UNSUPPORTED;
+  auto layout_of = [&](const TcChoice& c) {
+    return c.fused ? fused_layout(M, N, K, variant, fused_tile_ts(c.idx))
+                   : split_layout(M, N, K, variant);
+  };
+  auto partial_of = [&](const TcChoice& c) {
+    return c.splits > 1 ? align256((size_t)c.splits * M * N * 4) : 0;
+  };
+  auto fits = [&](const TcChoice& c) {
+    const size_t need = layout_of(c).total + partial_of(c);
+    return need == 0 || (ws && ws_bytes >= need && !(reinterpret_cast<uintptr_t>(ws) & 255));
+  };
+  if (!fits(ch)) {
+    // an automatic schedule gives up K slices for a workspace that holds the
+    // compact one (the allocation-free entry point's scratch, or a buffer
+    // sized by the parts alone)
+    if (tile >= 0 || (cfg && cfg->split_k > 0)) return HBSG_ERR_WORKSPACE;
+    tc_pick_compact(M, N, K, variant, sms, !(trans_a || trans_b) && fusable, &ch);
+    if (!fits(ch)) return HBSG_ERR_WORKSPACE;
+  }
   const int tc = ch.idx, splits = ch.splits;
-  const SplitLayout L = ch.fused ? fused_layout(M, N, K, variant, fused_tile_ts(tc))
-                                 : split_layout(M, N, K, variant);
-  const size_t partial_bytes = splits > 1 ? align256((size_t)splits * M * N * 4) : 0;
-  if (L.total + partial_bytes > 0 &&
-      (!ws || ws_bytes < L.total + partial_bytes || (reinterpret_cast<uintptr_t>(ws) & 255)))
-    return HBSG_ERR_WORKSPACE;
+  const SplitLayout L = layout_of(ch);
   uint8_t* w = static_cast<uint8_t*>(ws);
   void* Ap = w + L.a_off;
   void* Bp = w + L.b_off;

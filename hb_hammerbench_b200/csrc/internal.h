@@ -162,6 +162,11 @@ static constexpr int kMaxDevices = 64;
 // no sm_100 device is current (or its ordinal is >= kMaxDevices).
 int current_device_sms(int* device_out);
 
+// Workspace of the compact schedule of such a call (see tc_pick_compact): the
+// least a call without a config runs in.
+size_t gemm_compact_workspace(int trans_a, int trans_b, int m, int n, int k, const float* a,
+                              long lda, const float* b, long ldb, int variant);
+
 // A per-device figure of a kernel that the runtime takes microseconds to work
 // out (resident CTAs or clusters, for its fixed block and shared memory),
 // asked for once per device: `query` runs until it gives a positive value.

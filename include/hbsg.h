@@ -134,7 +134,9 @@ int hbsg_gemm_ex(int trans_a, int trans_b, int m, int n, int k,
                  float* c, int64_t ldc, int variant, const hbsg_config* cfg,
                  void* workspace, size_t workspace_bytes, hbsg_stream_t stream);
 
-/* Workspace bytes for hbsg_gemm / hbsg_gemm_ex on the current device. The
+/* Workspace bytes for hbsg_gemm / hbsg_gemm_ex on the current device. A call
+ * without a tile or split_k of its own that gets less than this, but enough
+ * for a schedule with fewer K slices (the compact schedule), runs that one. The
  * split-BF16 schedule, and so its K-slice partial buffer, depends on the
  * device's SM count: with no sm_100 device current the split-BF16 forms
  * report 0 (and the product call itself returns HBSG_ERR_NO_DEVICE). */
@@ -222,8 +224,8 @@ int hbsg_gemm_grouped(int count, const hbsg_problem* problems, int variant,
  * the library: HBSG_NOALLOC_SCRATCH_BYTES (16 MiB) of device memory that
  * every GPU which loads the library holds until the process exits.
  *
- *   - Problems whose workspace (hbsg_gemm_workspace_size_for on the same
- *     operands, no config) exceeds HBSG_NOALLOC_SCRATCH_BYTES are
+ *   - Problems whose least workspace (the compact schedule's, below)
+ *     exceeds HBSG_NOALLOC_SCRATCH_BYTES are
  *     rejected with HBSG_ERR_WORKSPACE before anything is launched. With a
  *     split pass, M = N = K = 1024 BF16X6 needs 12.6 MB and fits; shapes the
  *     library serves with a fused-split tile need only the K-slice partials
