@@ -443,9 +443,9 @@ def run_ours(args) -> None:
                 "frac_of_sustained": achieved / peaks["bf16_tflops_sustained"],
                 "kernel_ms": avg_kernel_ms,
                 "effective_fp32_tflops_of_kernel": flops / (avg_kernel_ms * 1e-3) / 1e12}
-        # per step: split passes (A, B; none when fused), row/column maxima
-        # (scaled forms), the product kernel
-        launches = args.steps * ((0 if fused else 2) + (2 if "scaled" in variant else 0) + 1)
+        # per step: the split pass over A and B (none when fused), the pass over
+        # the row/column maxima (scaled forms), the product kernel
+        launches = args.steps * ((0 if fused else 1) + (1 if "scaled" in variant else 0) + 1)
     else:
         roof = _ffma_roofline(statistics.mean(kern_ms), flops, fp32, n)
         launches = args.steps
