@@ -320,7 +320,8 @@ __device__ __forceinline__ void tc_fused_body(const Tiles& tiles, const TcRun& r
   const uint32_t base = (raw + 1023u) & ~1023u;
   uint8_t* smem = smem_raw + (base - raw);
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + S::kBarOff);
-  uint64_t* full = bars;                     // leader: both CTAs' converters filled the stage
+  uint64_t* full = bars;                     // each CTA: its converters filled the stage (leader:
+                                             // and the peer's, passed on by the peer's warp 0)
   uint64_t* empty = bars + STAGES;           // each CTA: the stage is free again
   uint64_t* tfull = bars + 2 * STAGES;       // each CTA: accumulator buffer ready
   uint64_t* tempty = bars + 2 * STAGES + 2;  // leader: both CTAs drained the buffer
@@ -341,7 +342,7 @@ __device__ __forceinline__ void tc_fused_body(const Tiles& tiles, const TcRun& r
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
-      mbar_init(&full[s], 2 * kConvWarps);
+      mbar_init(&full[s], leader ? kConvWarps + 1 : kConvWarps);
       mbar_init(&empty[s], 1);
     }
     for (int b = 0; b < 2; ++b) {
@@ -417,6 +418,32 @@ __device__ __forceinline__ void tc_fused_body(const Tiles& tiles, const TcRun& r
           }
         }
       }
+    } else if (lane == 0) {
+      // Peer CTA: tell the leader of each filled stage, one remote arrive per
+      // k-tile. (The converter warps arrived there themselves before: an
+      // arrive with release at cluster scope holds its warp until the part
+      // writes are visible to the pair, and the peer's slowest converter spent
+      // 2700 cycles per k-tile to the leader's 1900; now both spend 1800.
+      // 256 x 256 x 2^20, 6 products: 918 -> 892 us. What bounds the k-tile's
+      // 2944 cycles is shared memory: the tensor core's operand reads alone
+      // take 1917 and the staging, its reads and the part writes 900 more.
+      // Deeper or separate staging rings, A boxes grouped over two k-tiles and
+      // L2 prefetch change nothing or cost 3-10 %: the converters wait 130
+      // cycles for their data.)
+      const uint32_t full_leader0 = map_to_rank(smem_u32(&full[0]), 0);
+      uint32_t it = 0;
+      bool ok = true;
+      for (int t = pair; t < num_tiles && ok; t += pairs) {
+        const int KT = tiles.get(t).KT;
+        for (int kt = 0; kt < KT; ++kt, ++it) {
+          const int s = it % STAGES;
+          if (!wait_bounded(&full[s], (it / STAGES) & 1, abort_flag, lim)) {
+            ok = false;
+            break;
+          }
+          mbar_arrive_remote(full_leader0 + 8u * s);
+        }
+      }
     }
   } else if (warp == 1) {
     // ---------------- TMA loader of the FP32 staging ring (both CTAs) ----------------
@@ -466,7 +493,6 @@ __device__ __forceinline__ void tc_fused_body(const Tiles& tiles, const TcRun& r
     // Warps 2 .. 2+kAWarps-1 convert A rows, the others B columns, so each
     // warp's unit loop is branch-free: all of a k-tile's loads are issued
     // first and the units' independent split chains overlap.
-    const uint32_t full_leader0 = map_to_rank(smem_u32(&full[0]), 0);
     const bool a_role = warp < 2 + S::kAWarps;
     const int tr = a_role ? threadIdx.x - 64 : threadIdx.x - 64 - 32 * S::kAWarps;
     constexpr int NA = S::kUnitsA;   // unit slots per A thread (the last may be partial)
@@ -564,8 +590,7 @@ __device__ __forceinline__ void tc_fused_body(const Tiles& tiles, const TcRun& r
         __syncwarp();
         if (lane == 0) {
           mbar_arrive(&sempty[ss]);  // the staging slot may be reloaded
-          if (leader) mbar_arrive(&full[s]);
-          else mbar_arrive_remote(full_leader0 + 8u * s);
+          mbar_arrive(&full[s]);
         }
       }
     }
