@@ -107,7 +107,16 @@ struct TcChoice {
   bool fused;  // idx indexes the fused table (else the tensor-core table)
   int idx;
   int splits, kts;
+  int whole = 0;   // > 0: only the tiles after the first `whole` are sliced
+  long sliced = 0;  // floats of one slice's partials then
 };
+
+// Bytes of a schedule's K-slice partials.
+static size_t partial_bytes(const TcChoice& c, int M, int N) {
+  if (c.splits <= 1) return 0;
+  const size_t floats = c.whole > 0 ? (size_t)c.sliced : (size_t)M * N;
+  return (c.splits * floats * 4 + 255) / 256 * 256;
+}
 
 // ---- automatic split-BF16 schedule ----
 // Estimated microseconds of a call on a tile with s K slices:
@@ -162,6 +171,26 @@ static double tile_us(const TileCost& c, double split_bytes, long tiles, int slo
   return t;
 }
 
+// Slices of the last, unfilled round alone: a grid of 1 to 4 full rounds and
+// some tiles more leaves most SMs idle for a whole tile's time at the end;
+// those tiles in s slices each fill the SMs in rounds of 1/s. Only their
+// partials are written and reduced. Whole tiles -> last round sliced, 6
+// products, us: 2048 x 2560 x 4096 274 -> 240, 1537 x 3333 x 4096 293 -> 267,
+// 2100 x 2500 x 3000 209 -> 188, 4096^3 726 -> 693, 19072 x 250 x 1024
+// 148 -> 108; 3 products 165 -> 146, 179 -> 163, 125 -> 115, 422 -> 395, 90 -> 82.
+// Past four rounds the round saved is under a fifth and the SM clock falls
+// with the load (power cap), so it is not tried.
+static double tail_us(const TileCost& c, double split_bytes, long tiles, int slots, int KT, int s,
+                      double tile_elems) {
+  const int per = (KT + s - 1) / s;
+  const int slices = (KT + per - 1) / per;
+  const long full = tiles / slots, rest = tiles - full * slots;
+  const double tail = (double)((rest * slices + slots - 1) / slots);
+  return c.fixed + c.split * split_bytes / 6e6 + c.wave * (full + tail) +
+         c.ktile * (full * (double)KT + tail * per) +
+         c.reduce * slices * rest * tile_elems * 8.0 / 1e7 + c.sliced + 3.0;
+}
+
 // Slice counts tried when the caller names none: each at least 8 k-tiles, and
 // no more than about two rounds of the slots.
 static const int kSliceCounts[] = {1, 2, 3, 4, 6, 8, 12, 16, 24, 37, 48, 74, 111, 148};
@@ -174,7 +203,7 @@ static void tc_pick_auto(int M, int N, int K, int variant, int sms, int req, boo
   const double per_elem = 4.0 + 2.0 * P;
   const bool scaled = scaled_of(variant);
   double best = 0.0;
-  int best_s = 1;
+  int best_s = 1, whole = 0;
   bool have = false;
   auto consider = [&](bool fused, int idx, const TileCost& c, int bm, int bn, int slots,
                       double split_bytes) {
@@ -189,8 +218,23 @@ static void tc_pick_auto(int M, int N, int K, int variant, int sms, int req, boo
         best_s = s;
         ch->fused = fused;
         ch->idx = idx;
+        whole = 0;
       }
       if (req > 0) break;
+    }
+    const long full = tiles / slots, rest = tiles - full * slots;
+    if (fused || req > 0 || full < 1 || full > 4 || rest == 0) return;
+    for (int s : {2, 3, 4, 6, 8}) {
+      if (KT / s < 8) break;
+      const double t = tail_us(c, split_bytes, tiles, slots, KT, s, (double)bm * bn);
+      if (t < best) {
+        best = t;
+        best_s = s;
+        ch->fused = false;
+        ch->idx = idx;
+        whole = (int)(full * slots);
+        ch->sliced = rest * bm * bn;
+      }
     }
   };
   for (int i = 0; i < tc_num_tiles(); ++i) {
@@ -208,6 +252,7 @@ static void tc_pick_auto(int M, int N, int K, int variant, int sms, int req, boo
                fused_tile_slots(f, sms), bytes);
     }
   }
+  ch->whole = whole;
   ch->splits = ch->fused ? fused_pick_splits(ch->idx, M, N, K, best_s, sms, &ch->kts)
                          : tc_pick_splits(ch->idx, M, N, K, best_s, sms, &ch->kts);
 }
@@ -227,6 +272,7 @@ static void tc_pick_compact(int M, int N, int K, int variant, int sms, bool fusa
   const double maxima = scaled_of(variant) ? opnds * 4.0 / kHbm : 0.0;
   double score = 0.0;
   ch->fused = false;
+  ch->whole = 0;
   ch->idx = tc_pick_tile(M, N, K, P, sms, 0, &score);
   ch->splits = tc_pick_splits(ch->idx, M, N, K, 0, sms, &ch->kts);
   if (!fusable || K <= 0 || score <= 0.0) return;
@@ -316,7 +362,7 @@ static size_t workspace_needed(int M, int N, int K, int batch, int variant, cons
   if (sms < 0) return 0;
   TcChoice ch;
   if (!tc_schedule(M, N, K, variant, cfg, sms, transposed, fusable == 1, &ch)) return 0;
-  const size_t partial = ch.splits > 1 ? align256((size_t)ch.splits * M * N * 4) : 0;
+  const size_t partial = partial_bytes(ch, M, N);
   return (ch.fused ? fused_layout(M, N, K, variant, fused_tile_ts(ch.idx))
                    : split_layout(M, N, K, variant)).total + partial;
 }
@@ -345,7 +391,7 @@ size_t gemm_compact_workspace(int trans_a, int trans_b, int m, int n, int k, con
   tc_pick_compact(m, n, k, variant, sms, fusable, &ch);
   return (ch.fused ? fused_layout(m, n, k, variant, fused_tile_ts(ch.idx))
                    : split_layout(m, n, k, variant)).total +
-         (ch.splits > 1 ? align256((size_t)ch.splits * m * n * 4) : 0);
+         partial_bytes(ch, m, n);
 }
 
 // Core dispatcher for one (possibly batched) GEMM.
@@ -411,11 +457,8 @@ static int gemm_dispatch(int trans_a, int trans_b, int M, int N, int K, const fl
     return c.fused ? fused_layout(M, N, K, variant, fused_tile_ts(c.idx))
                    : split_layout(M, N, K, variant);
   };
-  auto partial_of = [&](const TcChoice& c) {
-    return c.splits > 1 ? align256((size_t)c.splits * M * N * 4) : 0;
-  };
   auto fits = [&](const TcChoice& c) {
-    const size_t need = layout_of(c).total + partial_of(c);
+    const size_t need = layout_of(c).total + partial_bytes(c, M, N);
     return need == 0 || (ws && ws_bytes >= need && !(reinterpret_cast<uintptr_t>(ws) & 255));
   };
   if (!fits(ch)) {
@@ -492,7 +535,7 @@ static int gemm_dispatch(int trans_a, int trans_b, int M, int N, int K, const fl
     if (e != cudaSuccess) return status_from(e);
     if (flags & HBSG_FLAG_SPLIT_ONLY) continue;
     e = tc_launch(tc, Ap, Bp, M, N, K, L.Kp, Cb, ldc, rowmax, colmax, raster, chunk, sms, 0, 0, st,
-                  splits, reinterpret_cast<float*>(w + L.total), after_split);
+                  splits, reinterpret_cast<float*>(w + L.total), after_split, ch.whole);
     if (e != cudaSuccess) return status_from(e);
   }
   return HBSG_OK;

@@ -59,7 +59,7 @@ cudaError_t tc_launch(int idx, const void* Ap, const void* Bp, int M, int N, int
                       float* C, long ldc, const uint32_t* rowmax, const uint32_t* colmax,
                       int raster, int chunk_k, int sms, int debug_skip_loads,
                       unsigned long long wait_limit_ns, cudaStream_t st, int splits = 1,
-                      float* partial = nullptr, bool after_split = false);
+                      float* partial = nullptr, bool after_split = false, int whole = 0);
 int tc_pick_splits(int idx, int M, int N, int K, int requested, int sms, int* kt_per_split);
 int ffma_pick_splits(int tile_idx, int M, int N, int K, int batch, int requested, int sms);
 // C[b] = sum over s of partial[b][s] (fixed order), partial rows of N floats.

@@ -42,6 +42,12 @@ struct TcParams {
   int kt_per_split;  // k-tiles per slice
   float* C;          // output, or the slice partials [splits][M][N] when splits > 1
   long ldc;
+  // splits > 1 and whole > 0: the first `whole` tiles are not sliced and go to
+  // out, only those of the last, unfilled round are (partials
+  // [splits][num_tiles - whole][tile rows][BN])
+  int whole;
+  float* out;
+  long ldo;
   const uint32_t* rowmax;  // null unless scaled
   const uint32_t* colmax;
 };
@@ -63,8 +69,10 @@ struct SingleTiles {
   // and writes its partial to C + s*M*N (row stride N).
   template <int TBM, int BN>
   __device__ __forceinline__ TileWork get_bn(int item) const {
-    const int slice = item / p->num_tiles;
-    const int t = item - slice * p->num_tiles;
+    const bool sliced = item >= p->whole;
+    const int part = p->num_tiles - p->whole;  // sliced tiles
+    const int slice = sliced ? (item - p->whole) / part : 0;
+    const int t = sliced ? item - slice * part : item;
     const int span = p->raster * p->tiles_n;
     const int g = t / span;
     const int first = g * p->raster;
@@ -81,8 +89,14 @@ struct SingleTiles {
     w.n0 = (in / gm) * BN;
     const int KT = p->Kp / kBK;
     w.kt0 = slice * p->kt_per_split;
-    w.KT = min(p->kt_per_split, KT - w.kt0);
-    if (p->splits > 1) {
+    w.KT = sliced ? min(p->kt_per_split, KT - w.kt0) : KT;
+    if (!sliced) {
+      w.C = p->out;
+      w.ldc = p->ldo;
+    } else if (p->whole > 0) {  // the tile's own block, addressed from (m0, n0)
+      w.C = p->C + ((long)slice * part + (t - p->whole)) * (TBM * BN) - ((long)w.m0 * BN + w.n0);
+      w.ldc = BN;
+    } else if (p->splits > 1) {
       w.C = p->C + (long)slice * p->M * p->N;
       w.ldc = p->N;
     } else {
@@ -97,9 +111,51 @@ struct SingleTiles {
 
 template <int BN, int TBM = kBM>
 struct SingleTilesBN : SingleTiles {
-  __device__ __forceinline__ int count() const { return p->num_tiles * p->splits; }
+  __device__ __forceinline__ int count() const {
+    return p->whole + (p->num_tiles - p->whole) * p->splits;
+  }
   __device__ __forceinline__ TileWork get(int t) const { return get_bn<TBM, BN>(t); }
 };
+
+// C = the sum of the slices, in order, for the tiles sliced on their own
+// (TcParams::whole > 0): one thread per 4 columns of a row. Bound by L2 (the
+// partials were just written there) and its launch: a few microseconds for
+// under a round of tiles.
+static constexpr int kTailThreads = 256;
+__global__ void __launch_bounds__(kTailThreads)
+    tail_reduce_kernel(const __grid_constant__ TcParams p, int bm, int bn, bool vec) {
+  const int per = bm * bn / (4 * kTailThreads);  // CTAs per tile
+  const int part = p.num_tiles - p.whole;
+  const int i = blockIdx.x / per;  // sliced tile
+  const int e = (blockIdx.x - i * per) * kTailThreads + threadIdx.x;
+  const int r = e / (bn / 4);
+  const int c = (e - r * (bn / 4)) * 4;
+  const int t = p.whole + i;
+  const int span = p.raster * p.tiles_n;
+  const int g = t / span;
+  const int first = g * p.raster;
+  const int gm = min(p.raster, p.tiles_m - first);
+  const int row = (first + (t - g * span) % gm) * bm + r;
+  const int col = ((t - g * span) / gm) * bn + c;
+  if (row >= p.M || col >= p.N) return;
+  const long block = (long)bm * bn;
+  const float* src = p.C + i * block + (long)r * bn + c;
+  float* dst = p.out + row * p.ldo + col;
+  if (vec) {  // N a multiple of 4: the quad lies inside
+    float4 s = __ldcs(reinterpret_cast<const float4*>(src));
+    for (int k = 1; k < p.splits; ++k) {
+      const float4 v = __ldcs(reinterpret_cast<const float4*>(src + k * part * block));
+      s = make_float4(s.x + v.x, s.y + v.y, s.z + v.z, s.w + v.w);
+    }
+    *reinterpret_cast<float4*>(dst) = s;
+  } else {
+    for (int j = 0; j < 4 && col + j < p.N; ++j) {
+      float s = src[j];
+      for (int k = 1; k < p.splits; ++k) s += src[k * part * block + j];
+      dst[j] = s;
+    }
+  }
+}
 
 template <int P, int BN, int STAGES, bool SCALED>
 __global__ void __launch_bounds__(320, 1)
@@ -375,7 +431,7 @@ cudaError_t tc_launch(int idx, const void* Ap, const void* Bp, int M, int N, int
                       float* C, long ldc, const uint32_t* rowmax, const uint32_t* colmax,
                       int raster, int chunk_k, int sms, int debug_skip_loads,
                       unsigned long long wait_limit_ns, cudaStream_t st, int splits,
-                      float* partial, bool after_split) {
+                      float* partial, bool after_split, int whole) {
   const TcEntry& e = kTcTiles[idx];
   CUtensorMap ma, mb;
   if (!tc_make_parts_map_impl(&ma, Ap, e.parts, M, Kp, kBM)) return cudaErrorInvalidValue;
@@ -396,6 +452,9 @@ cudaError_t tc_launch(int idx, const void* Ap, const void* Bp, int M, int N, int
   p.kt_per_split = kts;
   p.C = p.splits > 1 ? partial : C;
   p.ldc = p.splits > 1 ? N : ldc;
+  p.whole = p.splits > 1 ? whole : 0;
+  p.out = C;
+  p.ldo = ldc;
   p.rowmax = rowmax;
   p.colmax = colmax;
   TcRun run;
@@ -404,7 +463,7 @@ cudaError_t tc_launch(int idx, const void* Ap, const void* Bp, int M, int N, int
   run.l2_keep = tc_l2_keep();
   run.debug_skip_loads = debug_skip_loads;
   run.wait_limit_ns = wait_limit_ns ? wait_limit_ns : kWaitLimitNs;
-  const long items = (long)p.num_tiles * p.splits;
+  const long items = p.whole + (long)(p.num_tiles - p.whole) * p.splits;
   int grid;
   if (e.pair) {
     // every pair must be resident at once (tiles are dealt statically)
@@ -419,6 +478,14 @@ cudaError_t tc_launch(int idx, const void* Ap, const void* Bp, int M, int N, int
   }
   cudaError_t err = e.launch(ma, mb, p, run, grid, st, rowmax != nullptr, after_split);
   if (err != cudaSuccess || p.splits == 1) return err;
+  if (p.whole > 0) {
+    const bool vec =
+        (N & 3) == 0 && (ldc & 3) == 0 && (reinterpret_cast<uintptr_t>(C) & 15) == 0;
+    const unsigned blocks =
+        (unsigned)((p.num_tiles - p.whole) * (tbm * e.bn / (4 * kTailThreads)));
+    tail_reduce_kernel<<<blocks, kTailThreads, 0, st>>>(p, tbm, e.bn, vec);
+    return cudaGetLastError();
+  }
   return splitk_reduce(partial, C, M, N, ldc, 0, p.splits, 1, sms, st);
 }
 
