@@ -73,4 +73,28 @@ HBSG_DEV bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
   return ok != 0;
 }
 
+// ---- row and column scales of the scaled split-BF16 forms --------------------
+// frexp exponent of max|x| from its FP32 bit pattern: the scale 2^-e the
+// split applied to that row or column (0 for zero, non-finite or absent).
+HBSG_DEV int pow2_exp_of_bits(uint32_t bits) {
+  const int E = (int)((bits >> 23) & 0xffu);
+  if (E == 0xff || bits == 0u) return 0;
+  if (E != 0) return E - 126;
+  int e;
+  frexpf(__uint_as_float(bits), &e);  // subnormal maximum
+  return e;
+}
+
+// x * 2^s for scales that are no normal float, |s| < 1000: the product is exact
+// in FP64, so the conversion back rounds once, as ldexpf does (and, unlike it,
+// is no call, which would hold the epilogue's registers at every use).
+HBSG_DEV float scale_pow2_wide(float x, int s) {
+  return __double2float_rn((double)x * __hiloint2double((1023 + s) << 20, 0));
+}
+
+HBSG_DEV float scale_pow2(float x, int s) {
+  return s >= -126 && s <= 127 ? x * __uint_as_float((uint32_t)(s + 127) << 23)
+                               : scale_pow2_wide(x, s);
+}
+
 }  // namespace hbsg

@@ -76,7 +76,9 @@ __global__ void __launch_bounds__(FfmaShape<BM, BN, BK, WM, WN, STAGES>::kThread
   }
 }
 
-// Fixed-order reduction of split-K partial slices: C = ((p0 + p1) + p2) + ...
+// Fixed-order reduction of split-K partial slices: C = ((p0 + p1) + p2) + ...,
+// times 2^(row exponent + column exponent) in the scaled split-BF16 forms, whose
+// slices are partial sums of the normalised operands.
 // One thread per V consecutive outputs of a row (V = 4 when N and C's rows
 // allow 16-byte access), the loads of 16 slices issued before their adds, so
 // the serial chain is the adds alone: the partials come from L2 and one load
@@ -90,20 +92,31 @@ struct ReduceVec<4> {
   static __device__ __forceinline__ T add(T a, T b) {
     return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w);
   }
+  static __device__ __forceinline__ T scale(T a, int er, const uint32_t* colmax) {
+    return make_float4(scale_pow2(a.x, er + pow2_exp_of_bits(colmax[0])),
+                       scale_pow2(a.y, er + pow2_exp_of_bits(colmax[1])),
+                       scale_pow2(a.z, er + pow2_exp_of_bits(colmax[2])),
+                       scale_pow2(a.w, er + pow2_exp_of_bits(colmax[3])));
+  }
 };
 template <>
 struct ReduceVec<1> {
   using T = float;
   static __device__ __forceinline__ T add(T a, T b) { return a + b; }
+  static __device__ __forceinline__ T scale(T a, int er, const uint32_t* colmax) {
+    return scale_pow2(a, er + pow2_exp_of_bits(colmax[0]));
+  }
 };
 
 static constexpr int kReduceThreads = 128;
 static constexpr int kReduceAhead = 16;
 
-template <int V>
+template <int V, bool SCALED>
 __global__ void __launch_bounds__(kReduceThreads)
     splitk_reduce_kernel(const float* __restrict__ partial, float* __restrict__ C, int M, int N,
-                         long ldc, long strideC, int splits, long total) {
+                         long ldc, long strideC, int splits, long total,
+                         const uint32_t* __restrict__ rowmax,
+                         const uint32_t* __restrict__ colmax) {
   using R = ReduceVec<V>;
   using T = typename R::T;
   const long idx = blockIdx.x * (long)kReduceThreads + threadIdx.x;
@@ -126,6 +139,7 @@ __global__ void __launch_bounds__(kReduceThreads)
     for (int u = 0; u < kReduceAhead; ++u) s = R::add(s, v[u]);
   }
   for (; k < splits; ++k) s = R::add(s, __ldcs(reinterpret_cast<const T*>(src + k * MN)));
+  if constexpr (SCALED) s = R::scale(s, pow2_exp_of_bits(rowmax[r]), colmax + col);
   *reinterpret_cast<T*>(C + b * strideC + r * ldc + col) = s;
 }
 
@@ -302,19 +316,18 @@ cudaError_t ffma_launch(int tile_idx, FfmaParams p, int batch, int sms, cudaStre
 }
 
 cudaError_t splitk_reduce(const float* partial, float* C, int M, int N, long ldc, long strideC,
-                          int splits, int batches, int sms, cudaStream_t st) {
+                          int splits, int batches, int sms, cudaStream_t st,
+                          const uint32_t* rowmax, const uint32_t* colmax) {
   (void)sms;
   const bool vec = (N & 3) == 0 && (ldc & 3) == 0 && (strideC & 3) == 0 &&
                    (reinterpret_cast<uintptr_t>(partial) & 15) == 0 &&
                    (reinterpret_cast<uintptr_t>(C) & 15) == 0;
   const long total = (long)batches * M * (vec ? N / 4 : N);
   const unsigned blocks = (unsigned)((total + kReduceThreads - 1) / kReduceThreads);
-  if (vec)
-    splitk_reduce_kernel<4><<<blocks, kReduceThreads, 0, st>>>(partial, C, M, N, ldc, strideC,
-                                                               splits, total);
-  else
-    splitk_reduce_kernel<1><<<blocks, kReduceThreads, 0, st>>>(partial, C, M, N, ldc, strideC,
-                                                               splits, total);
+  auto kernel = rowmax ? (vec ? splitk_reduce_kernel<4, true> : splitk_reduce_kernel<1, true>)
+                       : (vec ? splitk_reduce_kernel<4, false> : splitk_reduce_kernel<1, false>);
+  kernel<<<blocks, kReduceThreads, 0, st>>>(partial, C, M, N, ldc, strideC, splits, total, rowmax,
+                                            colmax);
   return cudaGetLastError();
 }
 

@@ -62,9 +62,12 @@ cudaError_t tc_launch(int idx, const void* Ap, const void* Bp, int M, int N, int
                       float* partial = nullptr, bool after_split = false, int whole = 0);
 int tc_pick_splits(int idx, int M, int N, int K, int requested, int sms, int* kt_per_split);
 int ffma_pick_splits(int tile_idx, int M, int N, int K, int batch, int requested, int sms);
-// C[b] = sum over s of partial[b][s] (fixed order), partial rows of N floats.
+// C[b] = sum over s of partial[b][s] (fixed order), partial rows of N floats;
+// with rowmax / colmax (scaled forms, one batch) the sum times its row's and
+// column's scale.
 cudaError_t splitk_reduce(const float* partial, float* C, int M, int N, long ldc, long strideC,
-                          int splits, int batches, int sms, cudaStream_t st);
+                          int splits, int batches, int sms, cudaStream_t st,
+                          const uint32_t* rowmax = nullptr, const uint32_t* colmax = nullptr);
 int tc_read_and_clear_device_error();
 int grouped_read_and_clear_device_error();
 int tc_chunk_ktiles(int parts, int chunk_k);

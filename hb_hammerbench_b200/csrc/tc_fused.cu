@@ -49,6 +49,7 @@ struct FusedTiles {
     if (p->splits > 1) {
       w.C = p->C + (long)slice * p->M * p->N;
       w.ldc = p->N;
+      w.slice = true;
     } else {
       w.C = p->C;
       w.ldc = p->ldc;
@@ -307,7 +308,7 @@ cudaError_t fused_launch(int idx, FusedParams p, int raster, int chunk_k, int sm
   cudaError_t err = e.launch(ma, mb, p, run, (int)(e.ts ? units : 2 * units), st, scaled,
                              after_split);
   if (err != cudaSuccess || p.splits == 1) return err;
-  return splitk_reduce(partial, C, p.M, p.N, ldc, 0, p.splits, 1, sms, st);
+  return splitk_reduce(partial, C, p.M, p.N, ldc, 0, p.splits, 1, sms, st, p.rowmax, p.colmax);
 }
 
 int fused_read_and_clear_device_error() {

@@ -637,7 +637,7 @@ __device__ __forceinline__ void tc_fused_body(const Tiles& tiles, const TcRun& r
         __syncwarp();
 #pragma unroll
         for (int i = lane; i < COLS; i += 32)
-          wexp[i] = pow2_exp_of_bits(w.colmax[min(col0 + i, w.N - 1)]);
+          wexp[i] = w.slice ? 0 : pow2_exp_of_bits(w.colmax[min(col0 + i, w.N - 1)]);
         __syncwarp();
       }
       store_rows_transposed<COLS, SCALED>(sum, w, w.m0 + kBM * (int)rank + 32 * q, col0, lane,

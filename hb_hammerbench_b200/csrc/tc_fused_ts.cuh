@@ -426,7 +426,8 @@ __device__ __forceinline__ void tc_fused_ts_body(const Tiles& tiles, const TcRun
       if constexpr (SCALED) {
         __syncwarp();
 #pragma unroll
-        for (int i = lane; i < BN; i += 32) wexp[i] = pow2_exp_of_bits(w.colmax[min(w.n0 + i, w.N - 1)]);
+        for (int i = lane; i < BN; i += 32)
+          wexp[i] = w.slice ? 0 : pow2_exp_of_bits(w.colmax[min(w.n0 + i, w.N - 1)]);
         __syncwarp();
       }
       store_rows_transposed<BN, SCALED>(sum, w, w.m0 + 32 * q, w.n0, lane, wexp);

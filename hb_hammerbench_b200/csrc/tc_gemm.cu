@@ -90,6 +90,7 @@ struct SingleTiles {
     const int KT = p->Kp / kBK;
     w.kt0 = slice * p->kt_per_split;
     w.KT = sliced ? min(p->kt_per_split, KT - w.kt0) : KT;
+    w.slice = sliced && p->splits > 1;
     if (!sliced) {
       w.C = p->out;
       w.ldc = p->ldo;
@@ -118,10 +119,12 @@ struct SingleTilesBN : SingleTiles {
 };
 
 // C = the sum of the slices, in order, for the tiles sliced on their own
-// (TcParams::whole > 0): one thread per 4 columns of a row. Bound by L2 (the
+// (TcParams::whole > 0), times the scaled forms' row and column scale: one
+// thread per 4 columns of a row. Bound by L2 (the
 // partials were just written there) and its launch: a few microseconds for
 // under a round of tiles.
 static constexpr int kTailThreads = 256;
+template <bool SCALED>
 __global__ void __launch_bounds__(kTailThreads)
     tail_reduce_kernel(const __grid_constant__ TcParams p, int bm, int bn, bool vec) {
   const int per = bm * bn / (4 * kTailThreads);  // CTAs per tile
@@ -141,18 +144,23 @@ __global__ void __launch_bounds__(kTailThreads)
   const long block = (long)bm * bn;
   const float* src = p.C + i * block + (long)r * bn + c;
   float* dst = p.out + row * p.ldo + col;
+  const int er = SCALED ? pow2_exp_of_bits(p.rowmax[row]) : 0;
+  auto scaled = [&](float x, int j) {
+    return SCALED ? scale_pow2(x, er + pow2_exp_of_bits(p.colmax[col + j])) : x;
+  };
   if (vec) {  // N a multiple of 4: the quad lies inside
     float4 s = __ldcs(reinterpret_cast<const float4*>(src));
     for (int k = 1; k < p.splits; ++k) {
       const float4 v = __ldcs(reinterpret_cast<const float4*>(src + k * part * block));
       s = make_float4(s.x + v.x, s.y + v.y, s.z + v.z, s.w + v.w);
     }
-    *reinterpret_cast<float4*>(dst) = s;
+    *reinterpret_cast<float4*>(dst) =
+        make_float4(scaled(s.x, 0), scaled(s.y, 1), scaled(s.z, 2), scaled(s.w, 3));
   } else {
     for (int j = 0; j < 4 && col + j < p.N; ++j) {
       float s = src[j];
       for (int k = 1; k < p.splits; ++k) s += src[k * part * block + j];
-      dst[j] = s;
+      dst[j] = scaled(s, j);
     }
   }
 }
@@ -483,10 +491,11 @@ cudaError_t tc_launch(int idx, const void* Ap, const void* Bp, int M, int N, int
         (N & 3) == 0 && (ldc & 3) == 0 && (reinterpret_cast<uintptr_t>(C) & 15) == 0;
     const unsigned blocks =
         (unsigned)((p.num_tiles - p.whole) * (tbm * e.bn / (4 * kTailThreads)));
-    tail_reduce_kernel<<<blocks, kTailThreads, 0, st>>>(p, tbm, e.bn, vec);
+    (rowmax ? tail_reduce_kernel<true> : tail_reduce_kernel<false>)<<<blocks, kTailThreads, 0, st>>>(
+        p, tbm, e.bn, vec);
     return cudaGetLastError();
   }
-  return splitk_reduce(partial, C, M, N, ldc, 0, p.splits, 1, sms, st);
+  return splitk_reduce(partial, C, M, N, ldc, 0, p.splits, 1, sms, st, rowmax, colmax);
 }
 
 // Default drain interval: every 2 k-tiles (64 of K) for the 6-product form,

@@ -257,24 +257,6 @@ struct TcShape {
   static_assert(BN % 16 == 0 && BN >= 64 && BN <= 256, "UMMA N");
 };
 
-// frexp exponent of max|x| from its FP32 bit pattern: the scale 2^-e the
-// split applied to that row or column (0 for zero, non-finite or absent).
-HBSG_DEV int pow2_exp_of_bits(uint32_t bits) {
-  const int E = (int)((bits >> 23) & 0xffu);
-  if (E == 0xff || bits == 0u) return 0;
-  if (E != 0) return E - 126;
-  int e;
-  frexpf(__uint_as_float(bits), &e);  // subnormal maximum
-  return e;
-}
-
-// x * 2^s for scales that are no normal float, |s| < 1000: the product is exact
-// in FP64, so the conversion back rounds once, as ldexpf does (and, unlike it,
-// is no call, which would hold the epilogue's registers at every use).
-HBSG_DEV float scale_pow2_wide(float x, int s) {
-  return __double2float_rn((double)x * __hiloint2double((1023 + s) << 20, 0));
-}
-
 // One output tile of work for the kernel body.
 struct TileWork {
   int prob;               // problem index (grouped launches; 0 otherwise)
@@ -289,6 +271,10 @@ struct TileWork {
   int KT;   // k-tiles in this work item
   const uint32_t* rowmax;  // scaled forms only
   const uint32_t* colmax;
+  // a K slice of its tile, stored as it is: the slices are summed before the
+  // scaled forms' 2^(row exponent + column exponent) is applied (one slice may
+  // exceed the FP32 range, or lose bits below it, where the whole sum does not)
+  bool slice = false;
   // FP32 operands, read by the fused-split body only (tc_fused.cuh): A is
   // M x K (row stride lda), B is K x N (row stride ldb)
   const float* A = nullptr;
@@ -316,7 +302,8 @@ struct TcRun {
 // shares, which cost the grouped product (tiles of K ~ 1000, so much more C
 // per FLOP) about 10 % of its time; with VW = 4 this measured 7.3 -> 6.6 ms
 // on 512 products of ~1000^3 (32-byte chunks over 4-lane groups: 6.7 ms).
-// Scaled forms apply 2^(row exponent + column exponent) first.
+// Scaled forms apply 2^(row exponent + column exponent) first (for a K slice,
+// TileWork::slice, 2^0: its column exponents in wexp are 0 as well).
 template <int COLS, bool SCALED, int VW = 4>
 HBSG_DEV void store_rows_transposed(float* sum, const TileWork& w, int row0, int col0, int lane,
                                     const int* wexp, int row_end = 0x7fffffff) {
@@ -324,7 +311,7 @@ HBSG_DEV void store_rows_transposed(float* sum, const TileWork& w, int row0, int
   constexpr int NCH = 32 / VW;  // chunks per 32-column block = lanes per group
   if constexpr (SCALED) {
     const int row = row0 + lane;
-    const int er = row < w.M ? pow2_exp_of_bits(w.rowmax[row]) : 0;
+    const int er = row < w.M && !w.slice ? pow2_exp_of_bits(w.rowmax[row]) : 0;
     // the range of er + wexp[j] over the warp's block: where every scale 2^s
     // is a normal float (all but rows and columns at the ends of the exponent
     // range), one shift and one multiply per value. With the range tested per
@@ -699,7 +686,7 @@ __device__ __forceinline__ void tc_body(const Tiles& tiles, const TcRun& run) {
         __syncwarp();
 #pragma unroll
         for (int i = lane; i < COLS; i += 32)
-          wexp[i] = pow2_exp_of_bits(w.colmax[min(col0 + i, w.N - 1)]);
+          wexp[i] = w.slice ? 0 : pow2_exp_of_bits(w.colmax[min(col0 + i, w.N - 1)]);
         __syncwarp();
       }
       // an M = 64 accumulator (tiles with at most 64 valid rows) holds rows

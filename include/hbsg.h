@@ -52,8 +52,8 @@ typedef struct hbsg_config {
     int tile;          /* tile-shape id, 1-based index into hbsg_tile_info (0 = heuristic) */
     int split_k;       /* K slices, reduced in fixed order. FFMA: 0/1 = none (keeps the one
                           sequential FMA chain per output), n > 1 = n slices. Split-BF16:
-                          0 = library heuristic (slices only when the output has too few
-                          tiles to fill the GPU), 1 = none, n > 1 = n slices. */
+                          0 = library heuristic (slices where the output's tiles, or those
+                          of its last round, leave SMs idle), 1 = none, n > 1 = n slices. */
     int raster_group;  /* tile rows per rasterisation group (0 = heuristic) */
     int chunk_k;       /* split-BF16: K elements accumulated on the tensor core before the
                           partial is added in FP32 registers (0 = heuristic) */
