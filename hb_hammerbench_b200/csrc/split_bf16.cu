@@ -20,8 +20,9 @@
 // each is either row-major along k (A, transposed B: "rows") or k x n (B,
 // transposed A: "columns", transposed through shared memory). Unscaled forms
 // take one launch. Scaled forms take two: the first finishes rows (one CTA
-// reads a row for its maximum and again, from the cache, for the split) and
-// reduces the column maxima, the second splits the columns. 3001 x 2503 x
+// reads a row for its maximum and again, from the cache, for the split; many
+// short rows see kShortRows) and reduces the column maxima, the second splits
+// the columns. 3001 x 2503 x
 // 3607 in the scaled 3-product form: 71 -> 48 us of split
 // work, 4 launches and a memset before. At 8192^3 the passes run at 6.1 TB/s.
 #include "internal.h"
@@ -33,10 +34,24 @@ static constexpr int kSplitThreads = 256;
 // Rows up to this long are finished by one CTA each (max and split); longer
 // ones are cut into chunks of this many k for the maximum.
 static constexpr int kRowChunk = 16384;
+// Many short rows (kShortRows: K up to kShortK, kShortMany rows or more) go to
+// groups of 4 to 64 lanes instead, which read a row once and keep up to
+// kRowUnits units of 8 k a lane in registers between its maximum and its split.
+// A CTA each left most of its threads, and most of the loads an SM can have in
+// flight, unused: whole 3-product calls of 65536 x 64, transposed B, CTA -> group,
+// K = 32 113 -> 18.5 us, 128 126 -> 31, 512 173 -> 90, 2048 336 -> 302 (6 products
+// 155 -> 19, 178 -> 38, 228 -> 115, 443 -> 398). Longer rows give each thread of a
+// CTA a unit or more: from K = 4096 on the groups lose 3-10 %, where only the
+// maxima are wanted already at 2048 (10000 x 64 x 2048 67.6 -> 74.9 us; at 1500
+// 65536 rows 265 -> 228), and fewer rows fit a few rounds of CTAs either way.
+static constexpr int kRowUnits = 4;
+static constexpr int kShortK = 2048;
+static constexpr int kShortMaxK = 1536;  // the same for the maxima alone
+static constexpr int kShortMany = 4096;
 static constexpr int kColRows = 64;  // k rows per CTA of the column maxima
 
 // One operand's share of a launch (blocks [first, first + blocks)).
-enum SplitRole { kRowSplit, kRowMaxSplit, kRowMax, kColMax, kColSplit };
+enum SplitRole { kRowSplit, kRowMaxSplit, kRowMax, kColMax, kColSplit, kShortRows };
 struct SplitJob {
   const float* X;  // rows: n x K with row stride ld; columns: K x n
   long ld;
@@ -83,8 +98,59 @@ HBSG_DEV float row_max(const float* __restrict__ row, int k0, int k1, float* red
   return block_max(mx, red);
 }
 
-template <int P, bool SCALED>
+// Lanes of a short row's group: a unit each up to a warp, kRowUnits each beyond.
+__host__ __device__ inline unsigned short_row_lanes(int Kp) {
+  const int units = Kp / 8;
+  unsigned g = 4;
+  while ((int)g < units && (g < 32 || (int)g * kRowUnits < units)) g *= 2;
+  return g;
+}
+
+// Short rows: their maximum and (with parts) their split, one group per row.
+template <int P>
+HBSG_DEV void split_short_rows(const SplitJob& j, unsigned block, float* red) {
+  const unsigned g = short_row_lanes(j.Kp), l = threadIdx.x & (g - 1);
+  const unsigned r = block * (kSplitThreads / g) + threadIdx.x / g;
+  const bool live = r < (unsigned)j.n;
+  const float* row = j.X + (long)(live ? r : 0) * j.ld;
+  float v[kRowUnits][8];
+  float mx = 0.0f;
+#pragma unroll
+  for (int u = 0; u < kRowUnits; ++u) {
+    const int k0 = (int)(u * g + l) * 8;
+    if (k0 < j.Kp) {  // (the padding past K loads as zeros)
+      split_a_load(row + k0, k0, j.K, v[u]);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) mx = fmaxf(mx, finite_abs(v[u][i]));
+    }
+  }
+  for (unsigned o = (g < 32 ? g : 32) / 2; o > 0; o >>= 1)
+    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+  if (g > 32) {  // two warps a row
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = mx;
+    __syncthreads();
+    mx = fmaxf(mx, red[(threadIdx.x >> 5) ^ 1]);
+  }
+  if (!live) return;
+  if (l == 0) j.mx[r] = __float_as_uint(mx);
+  if (!j.parts) return;
+  const SplitScale sc = split_scale(exp_from_maxbits(__float_as_uint(mx)));
+  const long plane = (long)j.n * j.Kp;
+#pragma unroll
+  for (int u = 0; u < kRowUnits; ++u) {
+    const int k0 = (int)(u * g + l) * 8;
+    if (k0 < j.Kp) split_a_store<P, true>(v[u], sc, j.parts + (long)r * j.Kp + k0, plane);
+  }
+}
+
+// SHORT: kernels that take kShortRows jobs (whose registers would cost the
+// others a resident CTA).
+template <int P, bool SCALED, bool SHORT>
 HBSG_DEV void split_job(const SplitJob& j, unsigned block, float (*tile)[65]) {
+  if (SHORT && j.role == kShortRows) {
+    split_short_rows<P>(j, block, tile[0]);
+    return;
+  }
   switch (j.role) {
     case kRowSplit: {  // 8 consecutive k per thread, 4 units a block apart
       const unsigned upr = (unsigned)j.Kp / 8;
@@ -157,13 +223,13 @@ HBSG_DEV void split_job(const SplitJob& j, unsigned block, float (*tile)[65]) {
   }
 }
 
-template <int P, bool SCALED>
+template <int P, bool SCALED, bool SHORT>
 __global__ void __launch_bounds__(kSplitThreads) split_kernel(const __grid_constant__ SplitJobs jobs) {
   __shared__ float tile[64][65];
   grid_dep_trigger();  // the next split launch or the product may set itself up
   grid_dep_wait();     // second launch: the first one's maxima
-  if (blockIdx.x < jobs.first1) split_job<P, SCALED>(jobs.job[0], blockIdx.x, tile);
-  else split_job<P, SCALED>(jobs.job[1], blockIdx.x - jobs.first1, tile);
+  if (blockIdx.x < jobs.first1) split_job<P, SCALED, SHORT>(jobs.job[0], blockIdx.x, tile);
+  else split_job<P, SCALED, SHORT>(jobs.job[1], blockIdx.x - jobs.first1, tile);
 }
 
 static long blocks_of(const SplitJob& j) {
@@ -171,6 +237,7 @@ static long blocks_of(const SplitJob& j) {
   switch (j.role) {
     case kRowSplit: return cdiv((long)j.n * (j.Kp / 8), 4 * kSplitThreads);
     case kRowMaxSplit: return j.n;
+    case kShortRows: return cdiv(j.n, kSplitThreads / short_row_lanes(j.Kp));
     case kRowMax: return (long)j.n * cdiv(j.K, kRowChunk);
     case kColMax: return cdiv(j.n, kSplitThreads) * cdiv(j.K, kColRows);
     default: return cdiv(j.n, 64) * cdiv(j.Kp, 64);
@@ -188,8 +255,11 @@ static cudaError_t launch_jobs(SplitJob* job, int n, int parts, bool scaled, cud
   auto flush = [&]() -> cudaError_t {
     if (total == 0) return cudaSuccess;
     const unsigned grid = (unsigned)total;
-    void (*k)(SplitJobs) = parts == 3 ? (scaled ? split_kernel<3, true> : split_kernel<3, false>)
-                                      : (scaled ? split_kernel<2, true> : split_kernel<2, false>);
+    void (*k)(SplitJobs) =
+        parts == 3 ? (scaled ? split_kernel<3, true, false> : split_kernel<3, false, false>)
+                   : (scaled ? split_kernel<2, true, false> : split_kernel<2, false, false>);
+    if (jobs.job[0].role == kShortRows || (taken > 1 && jobs.job[1].role == kShortRows))
+      k = parts == 3 ? split_kernel<3, true, true> : split_kernel<2, true, true>;
     const cudaError_t e = launch_after(k, grid, kSplitThreads, 0, st, *launched, jobs);
     *launched = e == cudaSuccess;
     total = 0;
@@ -226,7 +296,8 @@ cudaError_t split_operands(const SplitOperand* ops, int n, int parts, bool scale
       j.role = o.columns ? kColSplit : kRowSplit;
       first[n1++] = j;
     } else if (!o.columns && o.K <= kRowChunk) {
-      j.role = kRowMaxSplit;
+      j.role = o.Kp <= (o.parts ? kShortK : kShortMaxK) && o.n >= kShortMany ? kShortRows
+                                                                            : kRowMaxSplit;
       first[n1++] = j;
     } else {
       const cudaError_t e = cudaMemsetAsync(o.mx, 0, sizeof(uint32_t) * (size_t)o.n, st);
