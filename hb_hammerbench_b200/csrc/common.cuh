@@ -79,10 +79,8 @@ HBSG_DEV bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
 HBSG_DEV int pow2_exp_of_bits(uint32_t bits) {
   const int E = (int)((bits >> 23) & 0xffu);
   if (E == 0xff || bits == 0u) return 0;
-  if (E != 0) return E - 126;
-  int e;
-  frexpf(__uint_as_float(bits), &e);  // subnormal maximum
-  return e;
+  // a subnormal maximum is bits * 2^-149, its top bit 31 - clz
+  return E != 0 ? E - 126 : -117 - __clz((int)bits);
 }
 
 // x * 2^s for scales that are no normal float, |s| < 1000: the product is exact

@@ -92,19 +92,21 @@ struct ReduceVec<4> {
   static __device__ __forceinline__ T add(T a, T b) {
     return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w);
   }
-  static __device__ __forceinline__ T scale(T a, int er, const uint32_t* colmax) {
-    return make_float4(scale_pow2(a.x, er + pow2_exp_of_bits(colmax[0])),
-                       scale_pow2(a.y, er + pow2_exp_of_bits(colmax[1])),
-                       scale_pow2(a.z, er + pow2_exp_of_bits(colmax[2])),
-                       scale_pow2(a.w, er + pow2_exp_of_bits(colmax[3])));
+  using Bits = uint4;
+  static __device__ __forceinline__ T scale(T a, int er, Bits c) {
+    return make_float4(scale_pow2(a.x, er + pow2_exp_of_bits(c.x)),
+                       scale_pow2(a.y, er + pow2_exp_of_bits(c.y)),
+                       scale_pow2(a.z, er + pow2_exp_of_bits(c.z)),
+                       scale_pow2(a.w, er + pow2_exp_of_bits(c.w)));
   }
 };
 template <>
 struct ReduceVec<1> {
   using T = float;
   static __device__ __forceinline__ T add(T a, T b) { return a + b; }
-  static __device__ __forceinline__ T scale(T a, int er, const uint32_t* colmax) {
-    return scale_pow2(a, er + pow2_exp_of_bits(colmax[0]));
+  using Bits = uint32_t;
+  static __device__ __forceinline__ T scale(T a, int er, Bits c) {
+    return scale_pow2(a, er + pow2_exp_of_bits(c));
   }
 };
 
@@ -128,6 +130,13 @@ __global__ void __launch_bounds__(kReduceThreads)
   const int r = (int)(row - (long)b * M);
   const long MN = (long)M * N;
   const float* src = partial + (long)b * splits * MN + (long)r * N + col;
+  // (the maxima's loads go out before the slices' and wait beside them)
+  uint32_t rbits = 0;
+  typename R::Bits cbits{};
+  if constexpr (SCALED) {
+    rbits = __ldg(rowmax + r);
+    cbits = __ldg(reinterpret_cast<const typename R::Bits*>(colmax + col));
+  }
   T s = *reinterpret_cast<const T*>(src);
   int k = 1;
   for (; k + kReduceAhead <= splits; k += kReduceAhead) {
@@ -139,7 +148,7 @@ __global__ void __launch_bounds__(kReduceThreads)
     for (int u = 0; u < kReduceAhead; ++u) s = R::add(s, v[u]);
   }
   for (; k < splits; ++k) s = R::add(s, __ldcs(reinterpret_cast<const T*>(src + k * MN)));
-  if constexpr (SCALED) s = R::scale(s, pow2_exp_of_bits(rowmax[r]), colmax + col);
+  if constexpr (SCALED) s = R::scale(s, pow2_exp_of_bits(rbits), cbits);
   *reinterpret_cast<T*>(C + b * strideC + r * ldc + col) = s;
 }
 

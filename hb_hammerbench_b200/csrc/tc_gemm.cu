@@ -144,9 +144,14 @@ __global__ void __launch_bounds__(kTailThreads)
   const long block = (long)bm * bn;
   const float* src = p.C + i * block + (long)r * bn + c;
   float* dst = p.out + row * p.ldo + col;
-  const int er = SCALED ? pow2_exp_of_bits(p.rowmax[row]) : 0;
+  uint32_t rbits = 0, cbits[4] = {};  // (loaded before the slices, to wait beside them)
+  if constexpr (SCALED) {
+    rbits = __ldg(p.rowmax + row);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) cbits[j] = __ldg(p.colmax + min(col + j, p.N - 1));
+  }
   auto scaled = [&](float x, int j) {
-    return SCALED ? scale_pow2(x, er + pow2_exp_of_bits(p.colmax[col + j])) : x;
+    return SCALED ? scale_pow2(x, pow2_exp_of_bits(rbits) + pow2_exp_of_bits(cbits[j])) : x;
   };
   if (vec) {  // N a multiple of 4: the quad lies inside
     float4 s = __ldcs(reinterpret_cast<const float4*>(src));
@@ -157,7 +162,9 @@ __global__ void __launch_bounds__(kTailThreads)
     *reinterpret_cast<float4*>(dst) =
         make_float4(scaled(s.x, 0), scaled(s.y, 1), scaled(s.z, 2), scaled(s.w, 3));
   } else {
-    for (int j = 0; j < 4 && col + j < p.N; ++j) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      if (col + j >= p.N) break;
       float s = src[j];
       for (int k = 1; k < p.splits; ++k) s += src[k * part * block + j];
       dst[j] = scaled(s, j);
