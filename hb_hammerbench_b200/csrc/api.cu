@@ -257,9 +257,9 @@ static void tc_pick_auto(int M, int N, int K, int variant, int sms, int req, boo
                          : tc_pick_splits(ch->idx, M, N, K, best_s, sms, &ch->kts);
 }
 
-// A schedule with fewer K slices, so less workspace: run where the automatic
-// choice's partials do not fit the caller's buffer, and the measure of which
-// problems the allocation-free entry point takes. Tiles by their score
+// A schedule with fewer K slices, so usually less workspace: run where the
+// automatic choice does not fit the caller's buffer, and with that one the
+// measure of which problems the allocation-free entry point takes. Tiles by their score
 // (split-pass tiles) or by waves of measured k-tile cycles (fused ones).
 static void tc_pick_compact(int M, int N, int K, int variant, int sms, bool fusable, TcChoice* ch) {
   constexpr double kRate = 1.6e15;  // BF16 MMA flop/s of a well-fed tile

@@ -165,8 +165,8 @@ static constexpr int kMaxDevices = 64;
 // no sm_100 device is current (or its ordinal is >= kMaxDevices).
 int current_device_sms(int* device_out);
 
-// Workspace of the compact schedule of such a call (see tc_pick_compact): the
-// least a call without a config runs in.
+// Workspace of the compact schedule of such a call (see tc_pick_compact). A call
+// without a config runs in this or in gemm_workspace_exact's, whichever it has.
 size_t gemm_compact_workspace(int trans_a, int trans_b, int m, int n, int k, const float* a,
                               long lda, const float* b, long ldb, int variant);
 

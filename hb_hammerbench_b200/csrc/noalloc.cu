@@ -72,12 +72,17 @@ extern "C" int hbsg_gemm_noalloc(int trans_a, int trans_b, int m, int n, int k, 
   if (variant < HBSG_BF16X3 || variant > HBSG_BF16X6_SCALED) return HBSG_ERR_UNSUPPORTED;
   if (m < 0 || n < 0 || k < 0) return HBSG_ERR_INVALID_ARG;
   if (m == 0 || n == 0) return HBSG_OK;
-  // Problems are taken by the compact schedule's workspace; hbsg_gemm_ex runs
-  // the automatic one where it fits the scratch as well. A fused-split schedule
-  // of an unscaled form may need no scratch at all (need == 0); argument and
-  // device errors are reported by hbsg_gemm_ex.
-  const size_t need = hbsg::gemm_compact_workspace(trans_a, trans_b, m, n, k, a, lda, b, ldb,
-                                                   variant);
+  // A problem is taken where the automatic or the compact schedule fits the
+  // scratch, and hbsg_gemm_ex runs the first of them that does. Neither is
+  // always the smaller: the automatic one may pick a fused tile, which keeps no
+  // parts of A, the compact one has fewer K slices. A fused-split schedule of an
+  // unscaled form may need no scratch at all (need == 0); argument and device
+  // errors are reported by hbsg_gemm_ex.
+  const size_t automatic = hbsg::gemm_workspace_exact(trans_a, trans_b, m, n, k, a, lda, b, ldb,
+                                                      variant, nullptr);
+  const size_t compact = hbsg::gemm_compact_workspace(trans_a, trans_b, m, n, k, a, lda, b, ldb,
+                                                      variant);
+  const size_t need = automatic < compact ? automatic : compact;
   if (need > HBSG_NOALLOC_SCRATCH_BYTES) return HBSG_ERR_WORKSPACE;
   void* scratch = nullptr;
   const int s2 = hbsg::noalloc_scratch(&scratch);

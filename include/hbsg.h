@@ -224,9 +224,10 @@ int hbsg_gemm_grouped(int count, const hbsg_problem* problems, int variant,
  * the library: HBSG_NOALLOC_SCRATCH_BYTES (16 MiB) of device memory that
  * every GPU which loads the library holds until the process exits.
  *
- *   - Problems whose least workspace (the compact schedule's, see
- *     hbsg_gemm_workspace_size) exceeds HBSG_NOALLOC_SCRATCH_BYTES are
- *     rejected with HBSG_ERR_WORKSPACE before anything is launched. With a
+ *   - Problems that exceed HBSG_NOALLOC_SCRATCH_BYTES in the automatic
+ *     schedule (hbsg_gemm_workspace_size_for on the same operands, no config)
+ *     and in the compact one (see hbsg_gemm_workspace_size) are rejected with
+ *     HBSG_ERR_WORKSPACE before anything is launched. With a
  *     split pass, M = N = K = 1024 BF16X6 needs 12.6 MB and fits; shapes the
  *     library serves with a fused-split tile need only the K-slice partials
  *     and, for the scaled forms, the row and column maxima.
