@@ -137,13 +137,27 @@ def resolve_config(m: int, n: int, k: int, variant, trans: bool, config):
     return autotune.lookup(m, n, k, name.lower())
 
 
+_first_fused = 0  # global id of the first fused-split tile
+
+
+def _fits_operands(config, operands) -> bool:
+    """Whether a looked-up schedule may run on these (address, row stride)
+    operands: a shape class holds sizes and views whose rows start off the
+    16-byte boundaries that the fused-split tiles' tensor maps need."""
+    global _first_fused
+    if not _first_fused:
+        _first_fused = min(t["tile"] for t in tiles() if t["fused"])
+    return config.get("tile", 0) < _first_fused or all(
+        p % 16 == 0 and ld % 4 == 0 for p, ld in operands)
+
+
 def gemm(a: torch.Tensor, b: torch.Tensor, c: torch.Tensor | None = None, variant="ffma",
          trans_a: bool = False, trans_b: bool = False, config=None,
          workspace: torch.Tensor | None = None) -> torch.Tensor:
     """c = op(a) @ op(b) for 2-D float32 CUDA tensors with unit inner stride.
     With trans_a, `a` holds A^T (k x m); with trans_b, `b` holds B^T (n x k).
     Without a config the autotuner's choice for the shape class is used when
-    one is known (resolve_config)."""
+    one is known (resolve_config) and takes these operands."""
     _check_f32_cuda("a", a)
     _check_f32_cuda("b", b)
     if a.dim() != 2 or b.dim() != 2 or a.stride(1) != 1 or b.stride(1) != 1:
@@ -162,9 +176,12 @@ def gemm(a: torch.Tensor, b: torch.Tensor, c: torch.Tensor | None = None, varian
     if c.dim() != 2 or c.stride(1) != 1 or tuple(c.shape) != (m, n):
         raise ValueError("c must be m x n with unit inner stride")
     v = _variant(variant)
-    cfgp = _config(resolve_config(m, n, k, variant, trans_a or trans_b, config))
     ta, tb = int(trans_a), int(trans_b)
     pa, lda, pb, ldb = a.data_ptr(), a.stride(0), b.data_ptr(), b.stride(0)
+    cfg = resolve_config(m, n, k, variant, trans_a or trans_b, config)
+    if config is None and cfg is not None and not _fits_operands(cfg, ((pa, lda), (pb, ldb))):
+        cfg = None
+    cfgp = _config(cfg)
     l = lib()
 
     def call(stream):
@@ -207,6 +224,10 @@ class GroupedPlan:
         if config is None and self.As and autotune.enabled():
             dims = [(a.shape[0], b.shape[1], a.shape[1]) for a, b in zip(self.As, self.Bs)]
             config = autotune.lookup_grouped(dims, _VARIANT_NAMES[self.variant])
+            if config is not None and not _fits_operands(
+                    config, ((p, ld) for q in self._arr for p, ld in ((q.a or 0, q.lda),
+                                                                      (q.b or 0, q.ldb)))):
+                config = None
         self.config = config
         self._cfg = _config(config)
         dev = self.As[0].device if self.As else torch.device("cuda")
