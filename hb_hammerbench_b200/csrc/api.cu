@@ -160,6 +160,9 @@ static const TileCost kFusedCost[] = {
     {5.3, 1.07, 3.23, 0.557, 0.79, 5.1},  // 6 products, A in TMEM, 128 x 128
     {5.1, 1.09, 3.24, 0.352, 0.63, 5.2},  // 3 products
 };
+static_assert(sizeof(kTcCost) == kNumTcTiles * sizeof(TileCost) &&
+                  sizeof(kFusedCost) == kNumFusedTiles * sizeof(TileCost),
+              "a cost for each tile");
 
 static double tile_us(const TileCost& c, double split_bytes, long tiles, int slots, int KT, int s,
                       double mn) {
@@ -191,9 +194,6 @@ static double tail_us(const TileCost& c, double split_bytes, long tiles, int slo
          c.reduce * slices * rest * tile_elems * 8.0 / 1e7 + c.sliced + 3.0;
 }
 
-// Slice counts tried when the caller names none: each at least 8 k-tiles, and
-// no more than about two rounds of the slots.
-static const int kSliceCounts[] = {1, 2, 3, 4, 6, 8, 12, 16, 24, 37, 48, 74, 111, 148};
 
 static void tc_pick_auto(int M, int N, int K, int variant, int sms, int req, bool fusable,
                          TcChoice* ch) {
@@ -205,10 +205,14 @@ static void tc_pick_auto(int M, int N, int K, int variant, int sms, int req, boo
   double best = 0.0;
   int best_s = 1, whole = 0;
   bool have = false;
+  // slice counts tried when the caller names none, up to one for every SM and
+  // with the quarters of that: each at least 8 k-tiles, and no more than about
+  // two rounds of the slots
+  const int slice_counts[] = {1, 2, 3, 4, 6, 8, 12, 16, 24, sms / 4, 48, sms / 2, 3 * sms / 4, sms};
   auto consider = [&](bool fused, int idx, const TileCost& c, int bm, int bn, int slots,
                       double split_bytes) {
     const long tiles = (long)((M + bm - 1) / bm) * ((N + bn - 1) / bn);
-    for (int s : kSliceCounts) {
+    for (int s : slice_counts) {
       if (req > 0) s = req;
       if (req <= 0 && s > 1 && (KT / s < 8 || tiles * s * 5 > 11L * slots)) break;
       const double t = tile_us(c, split_bytes, tiles, slots, KT, s < KT ? s : KT, mn);

@@ -48,6 +48,10 @@ struct SplitOperand {
 // launch_after).
 cudaError_t split_operands(const SplitOperand* ops, int n, int parts, bool scaled,
                            cudaStream_t st, bool* launched);
+// Entries of the split-pass and fused tile tables; the schedule's cost tables
+// (api.cu) have one row for each, in the same order.
+static constexpr int kNumTcTiles = 10;
+static constexpr int kNumFusedTiles = 8;
 int tc_num_tiles();
 bool tc_tile_info(int idx, hbsg_tile_info* out);
 int tc_tile_parts(int idx);

@@ -193,16 +193,16 @@ struct FusedEntry {
 // these only), then the A-in-TMEM tiles
 static const FusedEntry kFused[] = {HBSG_FUSED_TILE_LIST(HBSG_FUSED_ENTRY)
                                     HBSG_FUSED_TS_TILE_LIST(HBSG_FUSED_TS_ENTRY)};
-static constexpr int kNumFused = sizeof(kFused) / sizeof(kFused[0]);
+static_assert(sizeof(kFused) == kNumFusedTiles * sizeof(FusedEntry), "table length");
 
-int fused_num_tiles() { return kNumFused; }
+int fused_num_tiles() { return kNumFusedTiles; }
 int fused_tile_parts(int idx) { return kFused[idx].parts; }
 int fused_tile_bn(int idx) { return kFused[idx].bn; }
 int fused_tile_bm(int idx) { return kFused[idx].bm; }
 int fused_tile_ts(int idx) { return kFused[idx].ts; }
 
 bool fused_tile_info(int idx, hbsg_tile_info* out) {
-  if (idx < 0 || idx >= kNumFused) return false;
+  if (idx < 0 || idx >= kNumFusedTiles) return false;
   out->variant_class = 1;
   out->bm = kFused[idx].bm;
   out->bn = kFused[idx].bn;

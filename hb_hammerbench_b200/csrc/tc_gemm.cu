@@ -304,7 +304,7 @@ static cudaError_t launch_tc_pair(const CUtensorMap& a, const CUtensorMap& b, co
 static const TcEntry kTcTiles[] = {HBSG_TC_TILE_LIST(HBSG_TC_ENTRY_COMMA)
                                    HBSG_TC_PAIR_ENTRY(3, 256, 4),   // 256 x 256 pair, 6 products
                                    HBSG_TC_PAIR_ENTRY(2, 256, 6)};  // 256 x 256 pair, 3 products
-static constexpr int kNumTcTiles = sizeof(kTcTiles) / sizeof(kTcTiles[0]);
+static_assert(sizeof(kTcTiles) == kNumTcTiles * sizeof(TcEntry), "table length");
 
 int tc_num_tiles() { return kNumTcTiles; }
 
