@@ -445,7 +445,7 @@ static int gemm_dispatch(int trans_a, int trans_b, int M, int N, int K, const fl
     p.K = K;
     p.splits = splits;
     p.raster = cfg && cfg->raster_group > 0 ? cfg->raster_group : 8;
-    return status_from(ffma_launch(tile, p, batch, sms, st, trans_a ? 1 : 0, trans_b ? 1 : 0));
+    return status_from(ffma_launch(tile, p, batch, st, trans_a ? 1 : 0, trans_b ? 1 : 0));
   }
 
   // ---- split-BF16 on the tensor cores ----

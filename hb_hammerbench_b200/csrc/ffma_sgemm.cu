@@ -157,7 +157,7 @@ __global__ void __launch_bounds__(kReduceThreads)
 
 struct FfmaEntry {
   int bm, bn, bk, wm, wn, stages;
-  int threads, smem, per_sm;
+  int threads, smem;
   cudaError_t (*launch)(const FfmaParams&, dim3, cudaStream_t, bool vec);
 };
 
@@ -203,7 +203,6 @@ static cudaError_t launch_ffma_trans(const FfmaParams& p, dim3 grid, cudaStream_
   FfmaEntry {                                                                           \
     BM, BN, BK, WM, WN, ST, FfmaShape<BM, BN, BK, WM, WN, ST>::kThreads,                \
         FfmaShape<BM, BN, BK, WM, WN, ST>::smem_bytes(false, false),                    \
-        FfmaShape<BM, BN, BK, WM, WN, ST>::kMinBlocks,                                  \
         &launch_ffma<BM, BN, BK, WM, WN, ST, PAIR>                                      \
   }
 
@@ -243,6 +242,10 @@ bool ffma_tile_info(int idx, hbsg_tile_info* out) {
 // all charged. 1536 x 1024 x 2048 takes 64 x 64 tiles (three per SM at most,
 // 150 us) rather than 128 x 128 (one on 96 of the SMs, 177 us); 4096^3 takes
 // 128 x 128 (2.24 ms). Transposed operands have kernels for two of the shapes.
+// `res` is the row-major layout's: with only B transposed two 64 x 64 tiles fit
+// an SM (88 KB, both staging rings), but charging it two at 46 TFLOP/s moves one
+// ragged shape in twenty to 128 x 128, and of nine such one gained (1664 x 1836 x
+// 3635 654 -> 624 us; 865 x 1398 x 352 33.1 -> 38.5, 2304 x 1386 x 1856 281 -> 309).
 int ffma_pick_tile(int M, int N, int K, int batch, int num_sms, bool trans) {
   struct Rate {
     int idx, res;
@@ -280,8 +283,7 @@ size_t ffma_workspace_bytes(int M, int N, int batch, int splits) {
   return splits > 1 ? (size_t)M * N * batch * splits * sizeof(float) : 0;
 }
 
-cudaError_t ffma_launch(int tile_idx, FfmaParams p, int batch, int sms, cudaStream_t st, int ta,
-                        int tb) {
+cudaError_t ffma_launch(int tile_idx, FfmaParams p, int batch, cudaStream_t st, int ta, int tb) {
   // transposed operands: 128 x 128 or 64 x 64 tiles (the closest of the two)
   if (ta || tb) {
     const FfmaEntry& big = kFfmaTiles[0];
@@ -321,13 +323,12 @@ cudaError_t ffma_launch(int tile_idx, FfmaParams p, int batch, int sms, cudaStre
     err = e.launch(p, grid, st, vec);
   }
   if (err != cudaSuccess || p.splits == 1) return err;
-  return splitk_reduce(p.partial, p.C, p.M, p.N, p.ldc, p.strideC, p.splits, batch, sms, st);
+  return splitk_reduce(p.partial, p.C, p.M, p.N, p.ldc, p.strideC, p.splits, batch, st);
 }
 
 cudaError_t splitk_reduce(const float* partial, float* C, int M, int N, long ldc, long strideC,
-                          int splits, int batches, int sms, cudaStream_t st,
-                          const uint32_t* rowmax, const uint32_t* colmax) {
-  (void)sms;
+                          int splits, int batches, cudaStream_t st, const uint32_t* rowmax,
+                          const uint32_t* colmax) {
   const bool vec = (N & 3) == 0 && (ldc & 3) == 0 && (strideC & 3) == 0 &&
                    (reinterpret_cast<uintptr_t>(partial) & 15) == 0 &&
                    (reinterpret_cast<uintptr_t>(C) & 15) == 0;
@@ -338,20 +339,6 @@ cudaError_t splitk_reduce(const float* partial, float* C, int M, int N, long ldc
   kernel<<<blocks, kReduceThreads, 0, st>>>(partial, C, M, N, ldc, strideC, splits, total, rowmax,
                                             colmax);
   return cudaGetLastError();
-}
-
-// Split count for the FFMA kernel: the requested count, or (0) enough K
-// slices to fill every SM when the output has too few tiles, keeping at least
-// 16 k-tiles (256 of K) per slice.
-int ffma_pick_splits(int tile_idx, int M, int N, int K, int batch, int requested, int sms) {
-  if (requested > 0) return requested;
-  const FfmaEntry& e = kFfmaTiles[tile_idx];
-  const long tiles = (long)((M + e.bm - 1) / e.bm) * ((N + e.bn - 1) / e.bn) * batch;
-  const long slots = (long)sms * e.per_sm;
-  if (tiles * 2 > slots) return 1;
-  const long by_k = K / (16 * e.bk) > 1 ? K / (16 * e.bk) : 1;
-  const long s = (slots + tiles - 1) / tiles;
-  return (int)(s < by_k ? s : by_k);
 }
 
 }  // namespace hbsg

@@ -29,8 +29,8 @@ int ffma_num_tiles();
 bool ffma_tile_info(int idx, hbsg_tile_info* out);
 int ffma_pick_tile(int M, int N, int K, int batch, int num_sms, bool trans);
 size_t ffma_workspace_bytes(int M, int N, int batch, int splits);
-cudaError_t ffma_launch(int tile_idx, FfmaParams p, int batch, int sms, cudaStream_t st,
-                        int ta = 0, int tb = 0);
+cudaError_t ffma_launch(int tile_idx, FfmaParams p, int batch, cudaStream_t st, int ta = 0,
+                        int tb = 0);
 
 // ---- split-BF16 family ----------------------------------------------------------
 // One operand of the split pass: n output rows of K elements, either stored
@@ -65,12 +65,11 @@ cudaError_t tc_launch(int idx, const void* Ap, const void* Bp, int M, int N, int
                       unsigned long long wait_limit_ns, cudaStream_t st, int splits = 1,
                       float* partial = nullptr, bool after_split = false, int whole = 0);
 int tc_pick_splits(int idx, int M, int N, int K, int requested, int sms, int* kt_per_split);
-int ffma_pick_splits(int tile_idx, int M, int N, int K, int batch, int requested, int sms);
 // C[b] = sum over s of partial[b][s] (fixed order), partial rows of N floats;
 // with rowmax / colmax (scaled forms, one batch) the sum times its row's and
 // column's scale.
 cudaError_t splitk_reduce(const float* partial, float* C, int M, int N, long ldc, long strideC,
-                          int splits, int batches, int sms, cudaStream_t st,
+                          int splits, int batches, cudaStream_t st,
                           const uint32_t* rowmax = nullptr, const uint32_t* colmax = nullptr);
 int tc_read_and_clear_device_error();
 int grouped_read_and_clear_device_error();

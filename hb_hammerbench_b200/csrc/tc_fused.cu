@@ -308,7 +308,7 @@ cudaError_t fused_launch(int idx, FusedParams p, int raster, int chunk_k, int sm
   cudaError_t err = e.launch(ma, mb, p, run, (int)(e.ts ? units : 2 * units), st, scaled,
                              after_split);
   if (err != cudaSuccess || p.splits == 1) return err;
-  return splitk_reduce(partial, C, p.M, p.N, ldc, 0, p.splits, 1, sms, st, p.rowmax, p.colmax);
+  return splitk_reduce(partial, C, p.M, p.N, ldc, 0, p.splits, 1, st, p.rowmax, p.colmax);
 }
 
 int fused_read_and_clear_device_error() {

@@ -502,7 +502,7 @@ cudaError_t tc_launch(int idx, const void* Ap, const void* Bp, int M, int N, int
         p, tbm, e.bn, vec);
     return cudaGetLastError();
   }
-  return splitk_reduce(partial, C, M, N, ldc, 0, p.splits, 1, sms, st, rowmax, colmax);
+  return splitk_reduce(partial, C, M, N, ldc, 0, p.splits, 1, st, rowmax, colmax);
 }
 
 // Default drain interval: every 2 k-tiles (64 of K) for the 6-product form,
