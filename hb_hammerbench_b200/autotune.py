@@ -19,7 +19,12 @@ and K. Cache file: $HBSG_AUTOTUNE_CACHE, else
 
 Defaults: the package ships the table this tuner produced on a B200
 (tuned_b200.json, regenerated with `python -m hb_hammerbench_b200.autotune
---ship`). lookup() answers from the user cache first, then from that table, so
+--ship`). An entry whose choice is neither its fastest candidate nor the
+library's within 2 % of it says why: "sustained" holds the times of the
+schedules in question at several shapes of the class ("sustained_shapes"),
+alternated four times in regions of half a second, long enough to reach the
+power cap that a candidate's few launches end before, and the choice is the
+one of least geometric mean. lookup() answers from the user cache first, then from that table, so
 the host interface (sgemm.gemm, sgemm.GroupedPlan) runs the tuner's choice
 for every tuned shape class when the caller passes no schedule; shapes of no
 tuned class keep the C library's heuristic. HBSG_AUTOTUNE=0 turns the lookup
