@@ -177,12 +177,13 @@ static double tile_us(const TileCost& c, double split_bytes, long tiles, int slo
 // Slices of the last, unfilled round alone: a grid of 1 to 4 full rounds and
 // some tiles more leaves most SMs idle for a whole tile's time at the end;
 // those tiles in s slices each fill the SMs in rounds of 1/s. Only their
-// partials are written and reduced. Whole tiles -> last round sliced, 6
-// products, us: 2048 x 2560 x 4096 274 -> 240, 1537 x 3333 x 4096 293 -> 267,
-// 2100 x 2500 x 3000 209 -> 188, 4096^3 726 -> 693, 19072 x 250 x 1024
-// 148 -> 108; 3 products 165 -> 146, 179 -> 163, 125 -> 115, 422 -> 395, 90 -> 82.
-// Past four rounds the round saved is under a fifth and the SM clock falls
-// with the load (power cap), so it is not tried.
+// partials are written and reduced. Best tile whole -> last round sliced, calls
+// without the host interface's table in long alternating runs, us: 6 products
+// 2048 x 2560 x 4096 277 -> 237, 1537 x 3333 x 4096 295 -> 262, 2100 x 2500 x 3000
+// 207 -> 186, 4096^3 713 -> 688, 19072 x 250 x 1024 117 -> 109; 3 products, the
+// first four, 163 -> 144, 179 -> 163, 123 -> 114, 408 -> 400. Past four rounds the
+// round saved is under a fifth and the SM clock falls with the load (power cap),
+// so it is not tried.
 static double tail_us(const TileCost& c, double split_bytes, long tiles, int slots, int KT, int s,
                       double tile_elems) {
   const int per = (KT + s - 1) / s;

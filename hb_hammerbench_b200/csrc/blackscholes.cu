@@ -27,7 +27,7 @@
 //     access each way (64 bytes per option). HBM-bound: 10M records 117 -> 96 us,
 //     6.6 TB/s;
 //   - separate arrays (s, strike, r, v, t in; call, put out): 28 bytes per
-//     option. Bound by the issue rate: 10M options 66 -> 58 us.
+//     option. Bound by the issue rate: 10M options 66 -> 55-59 us by box.
 // Each thread prices two options, with packed two-lane arithmetic.
 #include <cuda_runtime.h>
 

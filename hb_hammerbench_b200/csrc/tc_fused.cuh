@@ -424,9 +424,10 @@ __device__ __forceinline__ void tc_fused_body(const Tiles& tiles, const TcRun& r
       // arrive with release at cluster scope holds its warp until the part
       // writes are visible to the pair, and the peer's slowest converter spent
       // 2700 cycles per k-tile to the leader's 1900; now both spend 1800.
-      // 256 x 256 x 2^20, 6 products: 918 -> 892 us. What bounds the k-tile's
-      // 2944 cycles is shared memory: the tensor core's operand reads alone
-      // take 1917 and the staging, its reads and the part writes 900 more.
+      // 256 x 256 x 2^20, 6 products: 918 -> 892 us. Of the k-tile's 2944
+      // cycles the MMAs alone, without conversion and loads, take 1917; the
+      // 208 KB that cross shared memory (TMA writes, the converters' reads and
+      // part writes, the operand reads) need 1664.
       // Deeper or separate staging rings, A boxes grouped over two k-tiles and
       // L2 prefetch change nothing or cost 3-10 %: the converters wait 130
       // cycles for their data.)
