@@ -70,6 +70,7 @@ struct GTiles {  // tile source for the tensor-core body (split pass run beforeh
   const CUtensorMap* maps;  // 2 per problem: A parts, B parts
   int n;
   __device__ __forceinline__ int count() const { return n; }
+  __device__ __forceinline__ bool slice(int) const { return false; }  // no K slices
   __device__ __forceinline__ TileWork get(int t) const {
     const int4 e = tiles[t];
     const GProblem& p = probs[e.x];

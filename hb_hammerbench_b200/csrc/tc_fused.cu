@@ -49,7 +49,6 @@ struct FusedTiles {
     if (p->splits > 1) {
       w.C = p->C + (long)slice * p->M * p->N;
       w.ldc = p->N;
-      w.slice = true;
     } else {
       w.C = p->C;
       w.ldc = p->ldc;
@@ -68,6 +67,7 @@ struct FusedTiles {
 template <int BN, int TBM = 2 * kBM>
 struct FusedTilesBN : FusedTiles {
   __device__ __forceinline__ TileWork get(int t) const { return get_bn<BN, TBM>(t); }
+  __device__ __forceinline__ bool slice(int) const { return p->splits > 1; }
 };
 
 template <int P, int BN, int STAGES, int SSTAGES, bool SCALED>

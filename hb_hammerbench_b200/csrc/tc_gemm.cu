@@ -90,7 +90,6 @@ struct SingleTiles {
     const int KT = p->Kp / kBK;
     w.kt0 = slice * p->kt_per_split;
     w.KT = sliced ? min(p->kt_per_split, KT - w.kt0) : KT;
-    w.slice = sliced && p->splits > 1;
     if (!sliced) {
       w.C = p->out;
       w.ldc = p->ldo;
@@ -116,6 +115,8 @@ struct SingleTilesBN : SingleTiles {
     return p->whole + (p->num_tiles - p->whole) * p->splits;
   }
   __device__ __forceinline__ TileWork get(int t) const { return get_bn<TBM, BN>(t); }
+  // whether work item t is one of several K slices of its tile
+  __device__ __forceinline__ bool slice(int t) const { return p->splits > 1 && t >= p->whole; }
 };
 
 // C = the sum of the slices, in order, for the tiles sliced on their own
