@@ -93,7 +93,22 @@ struct ReduceVec<4> {
     return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w);
   }
   using Bits = uint4;
-  static __device__ __forceinline__ T scale(T a, int er, Bits c) {
+  static __device__ __forceinline__ T scale(T a, uint32_t row, Bits c) {
+    // a finite, normal maximum's exponent is E - 126: all but the ends of the
+    // range take 2^(Er + Ec - 252) from the bits
+    const uint32_t e = row >> 23, e0 = e + (c.x >> 23), e1 = e + (c.y >> 23), e2 = e + (c.z >> 23),
+                   e3 = e + (c.w >> 23);
+    if (min(e, min(min(c.x, c.y), min(c.z, c.w)) >> 23) >= 1 &&
+        min(min(e0, e1), min(e2, e3)) > 125 && max(max(e0, e1), max(e2, e3)) <= 379 &&
+        max(row, max(max(c.x, c.y), max(c.z, c.w))) < 0x7f800000u)
+      return make_float4(a.x * __uint_as_float((e0 - 125) << 23),
+                         a.y * __uint_as_float((e1 - 125) << 23),
+                         a.z * __uint_as_float((e2 - 125) << 23),
+                         a.w * __uint_as_float((e3 - 125) << 23));
+    return scale_any(a, row, c);
+  }
+  static __device__ __noinline__ T scale_any(T a, uint32_t row, Bits c) {
+    const int er = pow2_exp_of_bits(row);
     return make_float4(scale_pow2(a.x, er + pow2_exp_of_bits(c.x)),
                        scale_pow2(a.y, er + pow2_exp_of_bits(c.y)),
                        scale_pow2(a.z, er + pow2_exp_of_bits(c.z)),
@@ -105,8 +120,8 @@ struct ReduceVec<1> {
   using T = float;
   static __device__ __forceinline__ T add(T a, T b) { return a + b; }
   using Bits = uint32_t;
-  static __device__ __forceinline__ T scale(T a, int er, Bits c) {
-    return scale_pow2(a, er + pow2_exp_of_bits(c));
+  static __device__ __forceinline__ T scale(T a, uint32_t row, Bits c) {
+    return scale_pow2(a, pow2_exp_of_bits(row) + pow2_exp_of_bits(c));
   }
 };
 
@@ -130,13 +145,6 @@ __global__ void __launch_bounds__(kReduceThreads)
   const int r = (int)(row - (long)b * M);
   const long MN = (long)M * N;
   const float* src = partial + (long)b * splits * MN + (long)r * N + col;
-  // (the maxima's loads go out before the slices' and wait beside them)
-  uint32_t rbits = 0;
-  typename R::Bits cbits{};
-  if constexpr (SCALED) {
-    rbits = __ldg(rowmax + r);
-    cbits = __ldg(reinterpret_cast<const typename R::Bits*>(colmax + col));
-  }
   T s = *reinterpret_cast<const T*>(src);
   int k = 1;
   for (; k + kReduceAhead <= splits; k += kReduceAhead) {
@@ -147,8 +155,14 @@ __global__ void __launch_bounds__(kReduceThreads)
 #pragma unroll
     for (int u = 0; u < kReduceAhead; ++u) s = R::add(s, v[u]);
   }
+  uint32_t rbits = 0;
+  typename R::Bits cbits{};
+  if constexpr (SCALED) {  // (beside the last slices' loads)
+    rbits = __ldg(rowmax + r);
+    cbits = __ldg(reinterpret_cast<const typename R::Bits*>(colmax + col));
+  }
   for (; k < splits; ++k) s = R::add(s, __ldcs(reinterpret_cast<const T*>(src + k * MN)));
-  if constexpr (SCALED) s = R::scale(s, pow2_exp_of_bits(rbits), cbits);
+  if constexpr (SCALED) s = R::scale(s, rbits, cbits);
   *reinterpret_cast<T*>(C + b * strideC + r * ldc + col) = s;
 }
 

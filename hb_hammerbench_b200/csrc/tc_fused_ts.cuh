@@ -422,16 +422,16 @@ __device__ __forceinline__ void tc_fused_ts_body(const Tiles& tiles, const TcRun
         if (lane == 0) mbar_arrive(&tempty[buf]);
       }
       if (!ok) break;
-      const bool slice = tiles.slice(t);
+      const int keep = tiles.slice(t) ? 0 : -1;
       int* wexp = col_exp + q * BN;
       if constexpr (SCALED) {
         __syncwarp();
 #pragma unroll
         for (int i = lane; i < BN; i += 32)
-          wexp[i] = slice ? 0 : pow2_exp_of_bits(w.colmax[min(w.n0 + i, w.N - 1)]);
+          wexp[i] = pow2_exp_of_bits(w.colmax[min(w.n0 + i, w.N - 1)]) & keep;
         __syncwarp();
       }
-      store_rows_transposed<BN, SCALED>(sum, w, w.m0 + 32 * q, w.n0, lane, wexp, slice);
+      store_rows_transposed<BN, SCALED>(sum, w, w.m0 + 32 * q, w.n0, lane, wexp, keep);
     }
   }
 

@@ -299,19 +299,20 @@ struct TcRun {
 // per FLOP) about 10 % of its time; with VW = 4 this measured 7.3 -> 6.6 ms
 // on 512 products of ~1000^3 (32-byte chunks over 4-lane groups: 6.7 ms).
 // Scaled forms apply 2^(row exponent + column exponent) first. A K slice is
-// stored as it is (2^0, and the column exponents in wexp are 0): the slices are
-// summed before the scale is applied, since one may exceed the FP32 range, or
-// lose bits below it, where the whole sum does not. (Tiles::slice tells from the
-// launch's parameters: a flag kept in TileWork over the accumulation made the
-// 256-wide tiles spill.)
+// stored as it is (keep 0 clears the row's exponent, and the caller those of the
+// columns in wexp; keep -1 otherwise): the slices are summed before the scale is
+// applied, since one may exceed the FP32 range, or lose bits below it, where the
+// whole sum does not. (Tiles::slice tells from the launch's parameters, and a
+// mask takes no branch: a flag kept in TileWork over the accumulation made the
+// 256-wide tiles spill, a branch here the fused ones.)
 template <int COLS, bool SCALED, int VW = 4>
 HBSG_DEV void store_rows_transposed(float* sum, const TileWork& w, int row0, int col0, int lane,
-                                    const int* wexp, bool slice, int row_end = 0x7fffffff) {
+                                    const int* wexp, int keep, int row_end = 0x7fffffff) {
   static_assert(VW == 4, "16-byte chunks (float4 stores)");
   constexpr int NCH = 32 / VW;  // chunks per 32-column block = lanes per group
   if constexpr (SCALED) {
     const int row = row0 + lane;
-    const int er = row < w.M && !slice ? pow2_exp_of_bits(w.rowmax[row]) : 0;
+    const int er = row < w.M ? pow2_exp_of_bits(w.rowmax[row]) & keep : 0;
     // the range of er + wexp[j] over the warp's block: where every scale 2^s
     // is a normal float (all but rows and columns at the ends of the exponent
     // range), one shift and one multiply per value. With the range tested per
@@ -679,7 +680,7 @@ __device__ __forceinline__ void tc_body(const Tiles& tiles, const TcRun& run) {
       }
       if (!ok) break;
       const int col0 = w.n0 + h * COLS;
-      const bool slice = tiles.slice(Tiles::kQueue ? t : t - (int)gridDim.x);
+      const int keep = tiles.slice(Tiles::kQueue ? t : t - (int)gridDim.x) ? 0 : -1;
       int* wexp = col_exp + (warp - 2) * COLS;  // this warp's column exponents
       if constexpr (SCALED) {
         // each warp stages the exponents of its own COLS columns (no barrier
@@ -687,16 +688,16 @@ __device__ __forceinline__ void tc_body(const Tiles& tiles, const TcRun& run) {
         __syncwarp();
 #pragma unroll
         for (int i = lane; i < COLS; i += 32)
-          wexp[i] = slice ? 0 : pow2_exp_of_bits(w.colmax[min(col0 + i, w.N - 1)]);
+          wexp[i] = pow2_exp_of_bits(w.colmax[min(col0 + i, w.N - 1)]) & keep;
         __syncwarp();
       }
       // an M = 64 accumulator (tiles with at most 64 valid rows) holds rows
       // 16 q .. 16 q + 15 in lanes 32 q .. 32 q + 15 of the warp's quadrant
       if (w.M - w.m0 <= 64)
-        store_rows_transposed<COLS, SCALED>(sum, w, w.m0 + 16 * q, col0, lane, wexp, slice,
+        store_rows_transposed<COLS, SCALED>(sum, w, w.m0 + 16 * q, col0, lane, wexp, keep,
                                             w.m0 + 16 * q + 16);
       else
-        store_rows_transposed<COLS, SCALED>(sum, w, w.m0 + 32 * q, col0, lane, wexp, slice);
+        store_rows_transposed<COLS, SCALED>(sum, w, w.m0 + 32 * q, col0, lane, wexp, keep);
     }
   }
 

@@ -229,17 +229,17 @@ __device__ __forceinline__ void tc_pair_body(const Tiles& tiles, const TcRun& ru
       }
       if (!ok) break;
       const int col0 = w.n0 + h * COLS;
-      const bool slice = tiles.slice(t);
+      const int keep = tiles.slice(t) ? 0 : -1;
       int* wexp = col_exp + (warp - 2) * COLS;
       if constexpr (SCALED) {
         __syncwarp();
 #pragma unroll
         for (int i = lane; i < COLS; i += 32)
-          wexp[i] = slice ? 0 : pow2_exp_of_bits(w.colmax[min(col0 + i, w.N - 1)]);
+          wexp[i] = pow2_exp_of_bits(w.colmax[min(col0 + i, w.N - 1)]) & keep;
         __syncwarp();
       }
       store_rows_transposed<COLS, SCALED>(sum, w, w.m0 + kBM * (int)rank + 32 * q, col0, lane,
-                                          wexp, slice);
+                                          wexp, keep);
     }
   }
 
