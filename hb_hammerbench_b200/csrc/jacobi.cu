@@ -264,6 +264,35 @@ __global__ void __launch_bounds__(kRingThreads)
   }
 }
 
+// Where the ring form is the faster, by GPU time of launches in a graph (vector
+// against ring form, us). It needs a march to stream along, z that fills three
+// quarters of its 128-wide tiles (512 x 512 x 32 39.3 against 41.7; 300 x 200 x
+// 260 33.0 against 32.9-35.0), and:
+//   - grids whose in- and output exceed what L2 holds of them (88 MB): 4 planes
+//     or more (20000 x 4 x 512 65.5 / 62.2, 5000 x 5 x 512 21.3 / 18.1; but 10000 x
+//     3 x 1024 51.5 / 54.8, 60000 x 1 x 256 34.3 / 45.0);
+//   - smaller ones of several z tiles: a second slab, where the vector form waits
+//     for 16 planes one by one (64 x 20 x 512 8.0 / 4.7, 300 x 14 x 256 7.0 / 5.1),
+//     from 17 planes on or with a CTA for every SM (64 x 14 x 512 6.8 / 7.0); on one
+//     slab each plane tile's halos cost more than the streaming saves (5000 x 1 x
+//     512 5.3 / 7.3, 148 x 10 x 4096 9.4 / 10.2);
+//   - smaller ones of a single z tile: from 17 planes on, where an SM takes no more
+//     CTAs in turn than of the vector form, whose slabs are longer (64 x 64 x 128
+//     5.5 / 4.9, 180 x 220 x 128 7.8 / 7.5; but 170 x 170 x 128, three CTAs an SM for
+//     two, 6.8 / 7.7, 1200 x 40 x 128 8.6 / 10.4, 300 x 300 x 100 12.3 / 14.7).
+static bool ring_wins(int nx, int ny, int nz, int sms) {
+  const long zt = ((long)nz + kRingZ - 1) / kRingZ, xt = ((long)nx + kXT - 1) / kXT,
+             yt = ((long)ny + kRingSlab - 1) / kRingSlab;
+  if (4L * nz < 3 * zt * kRingZ || xt > 65535 || yt > 65535) return false;
+  if ((long)nx * ny * nz > 11000000L) return ny >= 4;
+  const long ctas = zt * xt * yt;
+  if (zt == 1) {
+    const long vector_ctas = xt * (((long)ny + kYSlab - 1) / kYSlab);
+    return ny > kYSlab && (ctas + sms - 1) / sms <= (vector_ctas + sms - 1) / sms;
+  }
+  return ny > kYSlab || (ny > kRingSlab && ctas >= sms);
+}
+
 static bool ring_map(CUtensorMap* map, const float* A0, int nx, int ny, int nz) {
   return tc_make_f32_map_3d(map, A0, nz, nx, ny, kTileZ, kTileX, 1);
 }
@@ -299,18 +328,7 @@ extern "C" int hbsg_jacobi(int c0, int c1, const float* A0, float* Anext, int nx
     return HBSG_ERR_UNSUPPORTED;
   const cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   const bool vec = (nz & 3) == 0 && ((reinterpret_cast<uintptr_t>(A0) | reinterpret_cast<uintptr_t>(Anext)) & 15) == 0;
-  // The ring form needs a march to stream along: from 17 planes on, where the
-  // vector form starts a second slab and waits for 16 planes one by one
-  // (64 x 96 x 512: 11.2 against 10.3 us), or enough CTAs for every SM. A grid of few
-  // planes stays with the vector form (64 x 8 x 512: 8.0 against 8.6 us with the
-  // tensor map's encoding), and so does one whose z leaves more than a quarter
-  // of the 128-wide tiles outside (512 x 512 x 32: 39.3 against 41.7 us; 300 x
-  // 200 x 260: 33.0 against 32.9-35.0 us).
-  const long ring_ctas = (long)((nz + kRingZ - 1) / kRingZ) * ((nx + kXT - 1) / kXT) *
-                         ((ny + kRingSlab - 1) / kRingSlab);
-  const bool ring = vec && (ny > kYSlab || ring_ctas >= sms) &&
-                    4L * nz >= 3 * (((long)nz + kRingZ - 1) / kRingZ * kRingZ) &&
-                    (nx + kXT - 1) / kXT <= 65535 && (ny + kRingSlab - 1) / kRingSlab <= 65535;
+  const bool ring = vec && ring_wins(nx, ny, nz, sms);
   CUtensorMap map;
   if (ring && ring_map(&map, A0, nx, ny, nz)) {
     static uint64_t mask = 0;

@@ -1,5 +1,7 @@
-"""Jacobi grids of at most 16 planes on each side of the second way into the
-ring form, a CTA (128 z x 8 x x 12 y) for every SM: one plane, a few, two slabs.
+"""Jacobi grids on each side of the rules that pick the ring form: 3 and 4 planes
+where the grid exceeds what L2 holds of it, 12, 13, 16 and 17 planes below that,
+one and several z tiles, and CTAs (128 z x 8 x x 12 y) around whole rounds of the
+SMs in either form.
 Bar: bit-exact against the oracle's host_jacobi, nothing written outside the
 grid.
 """
@@ -10,12 +12,26 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("nx,ny,nz", [
-    (1176, 1, 128), (1184, 1, 128), (1177, 1, 128), (1200, 2, 124),  # 147, 148, 148, 150 CTAs
-    (128, 12, 1280), (113, 12, 1280), (112, 12, 1280),               # 160, 150, 140
-    (592, 13, 128), (588, 16, 100), (75, 5, 2000),                   # 148, 148, 160
+    (1184, 1, 128), (1200, 2, 124), (150, 12, 512),     # one slab
+    (150, 13, 512), (64, 13, 512), (64, 17, 260),       # second slab; under a CTA an SM
+    (296, 13, 256), (295, 16, 228), (280, 16, 256),     # 148, 148 and 140 CTAs
+    (592, 17, 128), (1184, 17, 124), (170, 170, 128),   # one z tile: 148, 296 and 330 CTAs,
+    (150, 250, 128), (160, 280, 100),                   # 399 and 480 (vector form: 304 and 360)
+    (148, 16, 4096), (1200, 18, 512),                   # several CTAs an SM
 ])
 @pytest.mark.parametrize("offset", [0, 1])
 def test_grids_bit_exact(oracle_mod, nx, ny, nz, offset):
+    _check(oracle_mod, nx, ny, nz, offset)
+
+
+# 11 000 000 points and one plane's row more
+@pytest.mark.parametrize("nx,ny,nz", [(3520, 3, 1024), (3584, 3, 1024), (2688, 4, 1024),
+                                      (21484, 4, 128), (21488, 4, 128), (300, 300, 124)])
+def test_grids_around_the_l2_line(oracle_mod, nx, ny, nz):
+    _check(oracle_mod, nx, ny, nz, 0)
+
+
+def _check(oracle_mod, nx, ny, nz, offset):
     import torch
 
     import hb_hammerbench_b200 as hb
