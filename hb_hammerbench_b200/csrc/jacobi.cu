@@ -26,7 +26,7 @@
 // instructions per point (the scalar form measured 66 % issue-active at 0.60
 // of the HBM roof on 512^3).
 //
-// Ring form (the vector form's condition, grids of many CTAs): the vector form
+// Ring form (the vector form's condition, grids that ring_wins): the vector form
 // has one plane's loads in flight per warp and waits for each (5.3 TB/s at 53 %
 // issue-active, DRAM traffic already the ideal 1.05 GB on 512^3). Here a
 // producer warp streams whole (10 rows x 136 z) plane tiles, halos included,
